@@ -10,6 +10,7 @@ from __future__ import annotations
 import argparse
 import concurrent.futures as cf
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -31,28 +32,38 @@ CUDA_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr
 # nvcc and the host objects use the system g++.
 HOST_CXX = shutil.which("g++") or "g++"
 
-LIB_SOURCES = ["rihvr_kernels.cu", "rihvr_solver.cu", "rihvr_params.cpp", "rihvr_noalloc.cu", "rihvr_image.cpp",
-               "rihvr_segment.cu", "rihvr_unet.cu", "rihvr_unet_tc.cu", "rihvr_frame.cu"]
+LIB_SOURCES = ["rihvr_fast_small.cu", "rihvr_fast_mid.cu", "rihvr_fast_640.cu", "rihvr_fast_large.cu",
+               "rihvr_kernels.cu", "rihvr_prox.cu", "rihvr_prox_f32.cu", "rihvr_prox_f16.cu",
+               "rihvr_prox_bf16.cu", "rihvr_lines.cu", "rihvr_tv3d.cu",
+               "rihvr_solver.cu", "rihvr_params.cpp", "rihvr_noalloc.cu", "rihvr_image.cpp",
+               "rihvr_segment.cu", "rihvr_unet.cu", "rihvr_unet_tc.cu",
+               "rihvr_frame.cu"]
 CLI_SOURCES = ["sparse_inverse_recon.cpp", "sparse_segmentation.cpp", "create_background.cpp"]
 # executable -> its sources (linked against the library)
 EXECUTABLES = {CLI: ["sparse_inverse_recon.cpp"], SEG_CLI: ["sparse_segmentation.cpp"],
                BG_CLI: ["create_background.cpp"]}
-HEADERS = ["rihvr_device.cuh", "rihvr_kernels.cuh", "rihvr_image.h", "rihvr_unet_tc.cuh", "rihvr_frame.cuh"]
+_INCLUDE = re.compile(r'^\s*#include "([^"]+)"', re.M)
 
 
 def _mtime(p: str) -> float:
     return os.path.getmtime(p) if os.path.exists(p) else -1.0
 
 
-def _newest_header() -> float:
-    hs = [os.path.join(CSRC, h) for h in HEADERS] + [os.path.join(INCLUDE, "rihvr.h")]
-    return max(_mtime(h) for h in hs)
+def _newest_input(path: str, seen: set) -> float:
+    """Newest of a source file and the project headers it includes."""
+    path = os.path.normpath(path)
+    if path in seen or not os.path.exists(path):
+        return -1.0
+    seen.add(path)
+    with open(path) as f:
+        names = _INCLUDE.findall(f.read())
+    return max([_mtime(path)] + [_newest_input(os.path.join(os.path.dirname(path), n), seen) for n in names])
 
 
 def _compile(src: str, force: bool, verbose: bool) -> str:
     path = os.path.join(CSRC, src)
     obj = os.path.join(BUILD, src + ".o")
-    if not force and _mtime(obj) > max(_mtime(path), _newest_header()):
+    if not force and _mtime(obj) > _newest_input(path, set()):
         return obj
     if src.endswith(".cu"):
         cmd = [NVCC, "-ccbin", HOST_CXX] + CUDA_FLAGS + ["-c", path, "-o", obj]

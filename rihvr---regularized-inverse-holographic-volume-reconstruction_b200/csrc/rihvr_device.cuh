@@ -174,17 +174,34 @@ __device__ __forceinline__ void small_dft(float2 (&a)[R]) {
     a[1] = cadd(m, s);
     a[2] = csub(m, s);
   } else {
-    float2 o[R];
-    static_for<R>([&](auto qc) {
-      constexpr int q = decltype(qc)::value;
-      float2 acc = a[0];
-      static_for<R - 1>([&](auto rc) {
-        constexpr int r = decltype(rc)::value + 1;
-        acc = cadd(acc, cmul_tw<(r * q) % R, R, INV>(a[r]));
-      });
-      o[q] = acc;
+    // odd primes by the symmetry of the kernel: with p_r = a_r + a_{R-r} and
+    // m_r = a_r - a_{R-r}, X_q and X_{R-q} are the sum and the difference of
+    // a_0 + sum_r cos(2 pi q r / R) p_r and -+ i sum_r sin(2 pi q r / R) m_r
+    static_assert(R == 5 || R == 7, "radix 2, 3, 4, 5 or 7");
+    constexpr int P = (R - 1) / 2;
+    float2 p[P], m[P];
+    const float2 a0 = a[0];
+    float2 s = a0;
+    static_for<P>([&](auto rc) {
+      constexpr int r = decltype(rc)::value;
+      p[r] = f2add(a[r + 1], a[R - 1 - r]);
+      m[r] = f2sub(a[r + 1], a[R - 1 - r]);
+      s = f2add(s, p[r]);
     });
-    static_for<R>([&](auto qc) { a[decltype(qc)::value] = o[decltype(qc)::value]; });
+    a[0] = s;
+    static_for<P>([&](auto qc) {
+      constexpr int q = decltype(qc)::value + 1;
+      float2 c = a0, d = make_float2(0.f, 0.f);
+      static_for<P>([&](auto rc) {
+        constexpr int r = decltype(rc)::value + 1;
+        // Tw carries the direction: im = -+ sin
+        constexpr float co = Tw<(q * r) % R, R, INV>::re, si = Tw<(q * r) % R, R, INV>::im;
+        c = f2fma(make_float2(co, co), p[r - 1], c);
+        d = r == 1 ? f2mul(make_float2(si, si), m[r - 1]) : f2fma(make_float2(si, si), m[r - 1], d);
+      });
+      a[q] = make_float2(c.x - d.y, c.y + d.x);      // c + i d
+      a[R - q] = make_float2(c.x + d.y, c.y - d.x);  // c - i d
+    });
   }
 }
 
