@@ -49,8 +49,7 @@ struct ProxArgs {
   // of every voxel, FP32 complex; null = one launch
   float2* gdx = nullptr;
   float2* gdy = nullptr;
-  // device copy of (beta, t, mu, s, thr); when set, the 2-D TV and L1 prox
-  // kernels read these instead of the values above, so that a captured
+  // device copy of (beta, t, mu, s, thr); when set, the prox kernels read these instead of the values above, so that a captured
   // launch picks up each attempt's step and momentum
   const float* dscal = nullptr;
 };
@@ -128,10 +127,8 @@ cudaError_t launch_materialize_x(int storage, const void* P, const void* Pprev, 
                                  long long n, cudaStream_t st);
 cudaError_t launch_store_volume(int storage, const float2* in, void* out, long long n, cudaStream_t st);
 cudaError_t launch_prox6_init(int storage, const ProxArgs& a, float2* X1, cudaStream_t st);
-cudaError_t launch_tv3_estimate(const float2* X1, const float2* gx, const float2* gy, const float2* gz, float2* Y,
-                                int W, int H, int Nz, float mu, cudaStream_t st);
-cudaError_t launch_tv3_dual(const float2* Y, float2* gx, float2* gy, float2* gz, int W, int H, int Nz, float s,
-                            cudaStream_t st);
+cudaError_t launch_tv3(const ProxArgs& a, float2* X1, float2* other, const float2** result, int* launches,
+                       cudaStream_t st);
 cudaError_t launch_prox6_finish(int storage, const ProxArgs& a, const float2* Y, int* nblocks_out,
                                 cudaStream_t st);
 

@@ -250,7 +250,7 @@ struct rihvr_ctx {
   // launch shapes chosen by the autotuner (0 = built-in choice)
   int tune_adj_chunks = 0, tune_tv_nseg = 0, tune_tv_kernel = 0;
   bool tuned = false;
-  float2 *X1 = nullptr, *gx = nullptr, *gy = nullptr, *gz = nullptr, *Y = nullptr;  // mode 6
+  float2 *X1 = nullptr, *Y = nullptr;  // mode 6
 
   double t = 0, alpha1 = 1, beta = 0, prev_f_resid = 0;
   int it = 0;
@@ -476,7 +476,7 @@ ProxArgs prox_args(rihvr_ctx* c, double t, bool device_scalars = false) {
   }
   // proximalFusedLasso2d shrinks only if l1 > 0 (:3715)
   if (c->mode == 7 && !(c->p.regularization_param > 0.f)) a.thr = 0.f;
-  if (device_scalars && c->mode != 6) a.dscal = c->scal_d;
+  if (device_scalars) a.dscal = c->scal_d;
   return a;
 }
 
@@ -493,15 +493,11 @@ int prox_volume(rihvr_ctx* c, double t, bool device_scalars = false) {
     KL(launch_prox_l1(c->storage, a, &nb, c->st));
   } else {
     KL(launch_prox6_init(c->storage, a, c->X1, c->st));
-    CK(cudaMemsetAsync(c->gx, 0, sizeof(float2) * c->V, c->st));
-    CK(cudaMemsetAsync(c->gy, 0, sizeof(float2) * c->V, c->st));
-    CK(cudaMemsetAsync(c->gz, 0, sizeof(float2) * c->V, c->st));
-    for (int i = 0; i < a.n_tv; ++i) {
-      KL(launch_tv3_estimate(c->X1, c->gx, c->gy, c->gz, c->Y, c->W, c->H, c->Nz, a.mu, c->st));
-      KL(launch_tv3_dual(c->Y, c->gx, c->gy, c->gz, c->W, c->H, c->Nz, a.s, c->st));
-    }
-    KL(launch_tv3_estimate(c->X1, c->gx, c->gy, c->gz, c->Y, c->W, c->H, c->Nz, a.mu, c->st));
-    KL(launch_prox6_finish(c->storage, a, c->Y, &nb, c->st));
+    const float2* est = nullptr;
+    int steps = 0;
+    CK(launch_tv3(a, c->X1, c->Y, &est, &steps, c->st));
+    c->launches += steps;
+    KL(launch_prox6_finish(c->storage, a, est, &nb, c->st));
   }
   return reduce_into(c, nb, SLOT_PROX);
 }
@@ -601,7 +597,7 @@ void drop_graphs(rihvr_ctx* c) {
     }
 }
 
-bool use_graphs(const rihvr_ctx* c) { return c->graphs && c->warm && !c->profiling && c->mode != 6; }
+bool use_graphs(const rihvr_ctx* c) { return c->graphs && c->warm && !c->profiling; }
 
 // Run `enqueue` as a CUDA graph (captured on first use) or eagerly.  A failed
 // capture turns graphs off for the context and runs the work eagerly.
@@ -1136,7 +1132,7 @@ std::atomic<int> g_batch_mode{0};
 // frames as one graph launch per iteration
 thread_local int g_batch_combined = 0;
 
-bool use_dev_loop(const rihvr_ctx* c) { return c->dev_loop && dev_loop_enabled() && use_graphs(c) && c->mode != 6; }
+bool use_dev_loop(const rihvr_ctx* c) { return c->dev_loop && dev_loop_enabled() && use_graphs(c); }
 
 // The three iteration graphs, one per position of P_k in the rotation
 // (iPrev, iCur, iNew) = (iCur + 2, iCur, iCur + 1) mod 3, built before any is
@@ -1451,9 +1447,6 @@ int create_ctx(const rihvr_params* params, int width, int height, int z_first, i
     rc = dalloc_t(c, &c->gdy, c->V);
   if (c->mode == 6) {
     if (rc == RIHVR_OK) rc = dalloc_t(c, &c->X1, c->V);
-    if (rc == RIHVR_OK) rc = dalloc_t(c, &c->gx, c->V);
-    if (rc == RIHVR_OK) rc = dalloc_t(c, &c->gy, c->V);
-    if (rc == RIHVR_OK) rc = dalloc_t(c, &c->gz, c->V);
     if (rc == RIHVR_OK) rc = dalloc_t(c, &c->Y, c->V);
   }
   c->partial_cap = max_partial_blocks(width, height, c->Nz);
