@@ -37,7 +37,7 @@ LIB_SOURCES = ["rihvr_fast_small.cu", "rihvr_fast_mid.cu", "rihvr_fast_640.cu", 
                "rihvr_prox_bf16.cu", "rihvr_lines.cu", "rihvr_tv3d.cu",
                "rihvr_solver.cu", "rihvr_params.cpp", "rihvr_noalloc.cu", "rihvr_image.cpp",
                "rihvr_segment.cu", "rihvr_unet.cu", "rihvr_unet_tc.cu",
-               "rihvr_frame.cu"]
+               "rihvr_unet_grad.cu", "rihvr_frame.cu"]
 CLI_SOURCES = ["sparse_inverse_recon.cpp", "sparse_segmentation.cpp", "create_background.cpp"]
 # executable -> its sources (linked against the library)
 EXECUTABLES = {CLI: ["sparse_inverse_recon.cpp"], SEG_CLI: ["sparse_segmentation.cpp"],

@@ -26,8 +26,8 @@
 // 16-channel slices, staging a 64 x 16 activation tile (zero outside the
 // volume, converted to BF16) and a 16 x Cout weight tile in shared memory.
 // The data gradient is the same kernel with the taps mirrored and the weight
-// matrix transposed; the weight gradient is a split-K GEMM (K = voxels) on the
-// same instruction with FP32 atomics into the gradient.
+// matrix transposed; the weight gradient is a GEMM over the voxels on the same
+// instruction (rihvr_unet_grad.cu).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -257,83 +257,6 @@ cudaError_t conv3(const float* X, int Cin, const __nv_bfloat16* Wt, int Cout, in
     case 48: return conv3_launch<6, 2>(X, Cin, Wt, Cout, co0, bias, Y, v, relu, mirror, st);
     case 64: return conv3_launch<8, 2>(X, Cin, Wt, Cout, co0, bias, Y, v, relu, mirror, st);
     default: return cudaErrorInvalidValue;
-  }
-}
-
-// dW[co][k][ci] += sum_v dY[v][co] X[v + off_k][ci] over a chunk of voxels:
-// M = Cout (up to 4 tiles of 16), N = 16 input channels, K = voxels.  Each
-// warp takes its own 16-voxel steps and adds its partial tile with atomics.
-// Grid: (voxel chunks, 27 taps, Cin / 16 slices).
-constexpr int kWgVox = 1024;  // voxels a block
-__global__ void __launch_bounds__(128) k_conv3_wgrad(const float* __restrict__ X, int Cin,
-                                                      const float* __restrict__ dY, int Cout,
-                                                      float* __restrict__ dW, Vol v) {
-  __shared__ __align__(16) __nv_bfloat16 At[4][64][16];  // [warp][co][voxel]
-  __shared__ __align__(16) __nv_bfloat16 Bt[4][16][16];  // [warp][ci][voxel]
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  const int k = blockIdx.y, s = blockIdx.z;
-  int dz, dy, dx;
-  tap_offsets(k, &dz, &dy, &dx);
-  const long long n = v.n();
-  const int mt = Cout / 16;
-  float acc[4][2][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.f;
-  const long long base = (long long)blockIdx.x * kWgVox;
-  for (int step = warp; step < kWgVox / 16; step += 4) {
-    const long long v0 = base + step * 16;
-    if (v0 >= n) break;
-    // dY tile, transposed: At[co][i] = dY[v0 + i][co]
-    for (int e = lane; e < 16 * Cout; e += 32) {
-      const int i = e / Cout, co = e - i * Cout;
-      const long long vv = v0 + i;
-      At[warp][co][i] = __float2bfloat16_rn(vv < n ? dY[vv * Cout + co] : 0.f);
-    }
-    // X tile at the tap, transposed: Bt[ci][i] = X[v0 + i + off][16 s + ci]
-    for (int e = lane; e < 256; e += 32) {
-      const int i = e >> 4, ci = e & 15;
-      const long long vv = v0 + i;
-      float x = 0.f;
-      if (vv < n) {
-        const int xx = (int)(vv % v.W) + dx, yy = (int)((vv / v.W) % v.H) + dy,
-                  zz = (int)(vv / ((long long)v.W * v.H)) + dz;
-        if (zz >= 0 && zz < v.D && yy >= 0 && yy < v.H && xx >= 0 && xx < v.W)
-          x = X[(((long long)zz * v.H + yy) * v.W + xx) * Cin + s * 16 + ci];
-      }
-      Bt[warp][ci][i] = __float2bfloat16_rn(x);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if (i >= mt) continue;
-      const unsigned a0 = *reinterpret_cast<const unsigned*>(&At[warp][i * 16 + g][2 * t]);
-      const unsigned a1 = *reinterpret_cast<const unsigned*>(&At[warp][i * 16 + g + 8][2 * t]);
-      const unsigned a2 = *reinterpret_cast<const unsigned*>(&At[warp][i * 16 + g][2 * t + 8]);
-      const unsigned a3 = *reinterpret_cast<const unsigned*>(&At[warp][i * 16 + g + 8][2 * t + 8]);
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const unsigned b0 = *reinterpret_cast<const unsigned*>(&Bt[warp][j * 8 + g][2 * t]);
-        const unsigned b1 = *reinterpret_cast<const unsigned*>(&Bt[warp][j * 8 + g][2 * t + 8]);
-        mma_bf16(acc[i][j], a0, a1, a2, a3, b0, b1);
-      }
-    }
-    __syncwarp();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    if (i >= mt) continue;
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int co = i * 16 + g + h * 8, ci = s * 16 + j * 8 + 2 * t;
-        float* d = dW + ((long long)co * 27 + k) * Cin + ci;
-        atomicAdd(d, acc[i][j][2 * h]);
-        atomicAdd(d + 1, acc[i][j][2 * h + 1]);
-      }
   }
 }
 
@@ -735,8 +658,7 @@ int conv_back(rihvr_unet* u, int li, const float* X, float* dY, float* dX) {
   const Vol v = u->lv[L.level];
   const long long n = v.n();
   k_relu_back<<<blocks_for(n * L.cout), 256, 0, u->st>>>(dY, u->act[li], n * L.cout);
-  dim3 grid((unsigned)((n + kWgVox - 1) / kWgVox), 27, L.cin / 16);
-  k_conv3_wgrad<<<grid, 128, 0, u->st>>>(X, L.cin, dY, L.cout, u->gw + L.w_off, v);
+  UCK(conv3_wgrad(X, L.cin, dY, L.cout, u->gw + L.w_off, v.D, v.H, v.W, u->st));
   k_bias_grad<<<(unsigned)std::min<long long>(1024, (n + 7) / 8), 256, 0, u->st>>>(dY, L.cout, n, u->gw + L.b_off);
   u->launches += 3;
   // the data gradient: output channels of the transposed weights in windows of 64

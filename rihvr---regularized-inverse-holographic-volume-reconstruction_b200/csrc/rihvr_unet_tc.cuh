@@ -48,5 +48,11 @@ bool tc_zmap_encode(TcMap* m, const __nv_bfloat16* X, int C, int D, int H, int W
 cudaError_t conv3_tcz(const TcMap& zmap, int Cin, const __nv_bfloat16* Wp, const float* bias, int Cout,
                       __nv_bfloat16* Y, int D, int H, int W, const TcHead* head, int* err, cudaStream_t st);
 
+// dW[co][tap][ci] += sum over voxels of dY[v][co] X[v + off][ci], FP32
+// channels-last operands rounded to BF16 (rihvr_unet_grad.cu); Cin a multiple
+// of 16, Cout 16, 32 or 64.
+cudaError_t conv3_wgrad(const float* X, int Cin, const float* dY, int Cout, float* dW, int D, int H, int W,
+                        cudaStream_t st);
+
 }  // namespace unet
 }  // namespace rihvr
