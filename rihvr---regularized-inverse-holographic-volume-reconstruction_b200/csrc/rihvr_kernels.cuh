@@ -76,6 +76,8 @@ size_t max_partial_blocks(int W, int H, int Nz);
 
 // square sizes whose adjoint column pass has the recurrence variant
 bool adj_recurrence_supported(int W, int H, int rec_mode = 2);
+// the variant (rec_mode) the adjoint column pass takes untuned for evenly spaced planes
+int adj_col_builtin(int W, int H, int Nz);
 // dz_uniform != 0: the planes are evenly spaced by dz_uniform (z_{k+1} - z_k,
 // exact in FP64), which lets the square fast sizes advance the transfer
 // function by a recurrence (rec_mode 1: twiddles regenerated each plane, three

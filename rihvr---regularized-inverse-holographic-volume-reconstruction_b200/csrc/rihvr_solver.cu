@@ -1472,6 +1472,7 @@ int create_ctx(const rihvr_params* params, int width, int height, int z_first, i
   c->dz_uniform = c->Nz > 1 ? zl[1] - zl[0] : 1.0;
   for (int k = 1; k + 1 < c->Nz && c->dz_uniform != 0; ++k)
     if (zl[(size_t)k + 1] - zl[(size_t)k] != c->dz_uniform) c->dz_uniform = 0;
+  if (c->dz_uniform != 0) c->tune_adj_rec = adj_col_builtin(width, height, c->Nz);
   if (cudaMemcpy(c->cturn, ct.data(), sizeof(double) * ct.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(c->zlist, zl.data(), sizeof(double) * zl.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemsetAsync(c->b, 0, sizeof(float) * c->HW, c->st) != cudaSuccess)
