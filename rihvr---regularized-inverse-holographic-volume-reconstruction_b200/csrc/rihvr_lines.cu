@@ -12,11 +12,11 @@
 // inputs of all its butterflies into registers (up to E elements) before a
 // barrier and writes the outputs after it.
 //
-// What bounds it: instruction issue (index arithmetic, the butterflies, and the
-// calls of the stage functions).  Radix-4/2/3/5/7 stages between two
+// What bounds it: instruction issue (90 instructions an element: butterflies,
+// twiddles, index arithmetic).  Radix-4/2/3/5/7 stages between two
 // shared-memory buffers, with an index division and a table load for every
 // twiddle, took five stages at n = 1280: 883 us for a row pass of 1280 x 1024
-// x 64 on a B200, 552 us here (200 us at the memory's rate).
+// x 64 on a B200, 508 us here (200 us at the memory's rate).
 #include <algorithm>
 #include <cstring>
 #include <map>
@@ -164,80 +164,97 @@ __device__ __forceinline__ void twiddle_inputs(float2 (&v)[R], const float2* __r
   }
 }
 
-// One stage of radix R over the block's lines.  split(b, m, magic_m, &c, &j):
-// line c and butterfly j of butterfly number b; load(c, i): element i of line
-// c; store(c, i, value): output element i of line c.  TO_SMEM: the outputs go to the
-// shared copy, which every thread must have read first.  LG, SG > 0: loads or
-// stores that carry the transfer function go in groups of that many, so that
-// the FP64 phases of all of them are not live at once.
-template <int R, int E, bool INV, bool FIRST, bool TO_SMEM, int LG, int SG, typename Split, typename Load, typename Store>
-__device__ __noinline__ void lstage(LStage s, int lines, const float2* __restrict__ tw, Split split, Load load,
-                                    Store store) {
-  constexpr int NB = butterflies(R, E);
-  float2 v[NB][R];
-  int cc[NB], jj[NB];
-  const int total = s.m * lines;
+// One stage of radix R over the block's lines, in two halves around the
+// barrier that ends the reads of the shared copy.  split(b, m, magic_m, &c,
+// &j): line c and butterfly j of butterfly number b; load(c, i): element i of
+// line c; store(c, i, value): output element i of line c.  A thread takes
+// butterflies threadIdx.x, + blockDim.x, ...; v holds their inputs one after
+// another.  G > 0: loads or stores that carry the transfer function go in
+// groups of that many, so that the FP64 phases of all of them are not live at
+// once.
+template <int R, int E, int G, typename Split, typename Load>
+__device__ __forceinline__ void stage_load(const LStage& s, int lines, Split split, Load load, float2 (&v)[E]) {
 #pragma unroll
-  for (int nb = 0; nb < NB; ++nb) {
+  for (int nb = 0; nb < butterflies(R, E); ++nb) {
     const int b = (int)threadIdx.x + nb * (int)blockDim.x;
-    cc[nb] = -1;
-    jj[nb] = 0;
-    if (b < total) {
-      split(b, s.m, s.magic_m, &cc[nb], &jj[nb]);
+    if (b < s.m * lines) {
+      int c, j;
+      split(b, s.m, s.magic_m, &c, &j);
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        v[nb][r] = load(cc[nb], jj[nb] + r * s.m);
-        if (LG > 0 && r % (LG > 0 ? LG : 1) == LG - 1) sched_fence();
+        v[nb * R + r] = load(c, j + r * s.m);
+        if (G > 0 && r % (G > 0 ? G : 1) == G - 1) sched_fence();
       }
     }
   }
-  if (TO_SMEM) __syncthreads();
+}
+
+template <int R, int E, int G, bool INV, bool FIRST, typename Split, typename Store>
+__device__ __forceinline__ void stage_store(const LStage& s, int lines, const float2* __restrict__ tw, Split split,
+                                            Store store, float2 (&v)[E]) {
 #pragma unroll
-  for (int nb = 0; nb < NB; ++nb) {
-    if (cc[nb] < 0) continue;
-    const int j = jj[nb];
-    int k = 0;
-    if (!FIRST) {
-      k = j - (int)__umulhi((unsigned)j, s.magic_ns) * s.ns;
-      twiddle_inputs<R, INV>(v[nb], tw, k * s.tstep);
-    }
-    reg_fft<R, INV>(v[nb]);
-    const int d = (j - k) * R + k;
+  for (int nb = 0; nb < butterflies(R, E); ++nb) {
+    const int b = (int)threadIdx.x + nb * (int)blockDim.x;
+    if (b < s.m * lines) {
+      int c, j, k = 0;
+      split(b, s.m, s.magic_m, &c, &j);
+      float2 a[R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      store(cc[nb], d + r * s.ns, v[nb][r]);
-      if (SG > 0 && r % (SG > 0 ? SG : 1) == SG - 1) sched_fence();
+      for (int r = 0; r < R; ++r) a[r] = v[nb * R + r];
+      if (!FIRST) {
+        k = j - (int)__umulhi((unsigned)j, s.magic_ns) * s.ns;
+        twiddle_inputs<R, INV>(a, tw, k * s.tstep);
+      }
+      reg_fft<R, INV>(a);
+      const int d = (j - k) * R + k;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        store(nb * R + r, c, d + r * s.ns, a[r]);
+        if (G > 0 && r % (G > 0 ? G : 1) == G - 1) sched_fence();
+      }
     }
   }
-  if (TO_SMEM) __syncthreads();
 }
 
 #define RIHVR_EACH_RADIX(X) X(16) X(15) X(12) X(10) X(9) X(8) X(7) X(6) X(5) X(4) X(3) X(2)
 
+// the barrier stands outside the switches: with one in every case, the
+// compiler merged the cases around it and spilled up to 4 KB a thread
 template <int E, bool INV, bool FIRST, bool TO_SMEM, int LG, int SG, typename Split, typename Load, typename Store>
 __device__ __forceinline__ void any_stage(const LStage& s, int lines, const float2* __restrict__ tw, Split split,
                                           Load load, Store store) {
-  // one function a radix: inlined into one switch, the twelve cases spilled
-  // (968 to 3920 bytes of stack a kernel), each alone fits 50 to 90 registers
+  float2 v[E];
   switch (s.r) {
-#define RIHVR_CASE(RR)                                                            \
-  case RR:                                                                        \
-    lstage<RR, E, INV, FIRST, TO_SMEM, LG, SG>(s, lines, tw, split, load, store); \
+#define RIHVR_CASE(RR)                                 \
+  case RR:                                             \
+    stage_load<RR, E, LG>(s, lines, split, load, v);   \
     break;
     RIHVR_EACH_RADIX(RIHVR_CASE)
 #undef RIHVR_CASE
     default:
       break;
   }
+  if (TO_SMEM) __syncthreads();
+  switch (s.r) {
+#define RIHVR_CASE(RR)                                                \
+  case RR:                                                            \
+    stage_store<RR, E, SG, INV, FIRST>(s, lines, tw, split, store, v); \
+    break;
+    RIHVR_EACH_RADIX(RIHVR_CASE)
+#undef RIHVR_CASE
+    default:
+      break;
+  }
+  if (TO_SMEM) __syncthreads();
 }
 
-// all stages: src(c, i) the global input, dst(c, i, value) the global
+// all stages: src(c, i) the global input, dst(q, c, i, value) the global
 // output, at(c, i) an element's place in the shared copy
 template <int E, bool INV, int LG = 0, int SG = 0, typename Split, typename Src, typename Dst, typename At>
 __device__ __forceinline__ void line_fft(const LPlan& p, int lines, const float2* __restrict__ tw, float2* sm,
                                          Split split, Src src, Dst dst, At at) {
   const auto from = [=](int c, int i) { return sm[at(c, i)]; };
-  const auto to = [=](int c, int i, float2 v) { sm[at(c, i)] = v; };
+  const auto to = [=](int, int c, int i, float2 v) { sm[at(c, i)] = v; };
   any_stage<E, INV, true, true, LG, 0>(p.s[0], lines, tw, split, src, to);
 #pragma unroll 1
   for (int i = 1; i + 1 < p.nst; ++i) any_stage<E, INV, false, true, 0, 0>(p.s[i], lines, tw, split, from, to);
@@ -314,7 +331,7 @@ __global__ void __launch_bounds__(kRowThreadsMax, 2)
         *j = b - *c * m;
       },
       [=](int c, int i) { return load_as<IN>(in, base + (size_t)(c * n + i)); },
-      [=](int c, int i, float2 v) { out[base + (size_t)(c * n + i)] = cscale(v, scale); },
+      [=](int, int c, int i, float2 v) { out[base + (size_t)(c * n + i)] = cscale(v, scale); },
       [=](int c, int i) { return c * ls + padded(i); });
 }
 
@@ -368,7 +385,7 @@ __global__ void __launch_bounds__(kColThreadsMax, 1)
           const unsigned i = (unsigned)(y * W + x0 + c);
           return cmul(__ldg(Rs + i), transfer(zz, __ldg(cturn + i), true));
         },
-        [=](int c, int y, float2 v) {
+        [=](int, int c, int y, float2 v) {
           if (x0 + c < W) Uz[(unsigned)(y * W + x0 + c)] = v;
         },
         ColAt{logc});
@@ -400,7 +417,7 @@ __global__ void __launch_bounds__(kColThreadsMax, 1)
         [=](int c, int y) {
           return x0 + c < W ? __ldg(Tz + (unsigned)(y * W + x0 + c)) : make_float2(0.f, 0.f);
         },
-        [=](int c, int y, float2 v) {
+        [=](int, int c, int y, float2 v) {
           if (x0 + c >= W) return;
           const float2 h = transfer(zz, __ldg(cturn + (unsigned)(y * W + x0 + c)), false);
           float2 a = acc[(y << logc) + c];
@@ -427,7 +444,7 @@ __global__ void __launch_bounds__(kColThreadsMax, 1)
   line_fft<kElems, INV>(
       p, 1 << logc, tw, gbuf, ColSplit{logc},
       [=](int c, int y) { return x0 + c < W ? in[(unsigned)(y * W + x0 + c)] : make_float2(0.f, 0.f); },
-      [=](int c, int y, float2 v) {
+      [=](int, int c, int y, float2 v) {
         if (x0 + c < W) out[(unsigned)(y * W + x0 + c)] = cscale(v, scale);
       },
       ColAt{logc});
