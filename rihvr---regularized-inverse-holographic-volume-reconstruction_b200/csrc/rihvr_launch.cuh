@@ -113,11 +113,12 @@ __device__ __forceinline__ ProxArgs resolve_scalars(const ProxArgs& a0) {
 }
 
 // Square roots of the objective's norm terms (L1 and TV sums) use the
-// hardware approximation (PTX sqrt.approx.f32, one instruction): they only
-// feed the reported objective, summed over millions of voxels in FP64.
+// hardware approximation in its flush-to-zero form (one instruction; a
+// magnitude below 1.1e-19 counts as 0): they only feed the reported objective,
+// summed over millions of voxels in FP64.
 __device__ __forceinline__ float norm_sqrt(float q) {
   float r;
-  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(q));
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(q));
   return r;
 }
 

@@ -49,11 +49,14 @@ __device__ __forceinline__ float2 tv_estimate(float2 xh, float2 gx, float2 gxr, 
   return f2fma(nmu, f2add(f2sub(gxr, gx), f2sub(gyd, gy)), xh);
 }
 
-// hardware reciprocal square root (PTX rsqrt.approx.f32), one instruction
-// wherever it is inlined
+// hardware reciprocal square root.  The flush-to-zero form is one instruction;
+// the other one scales subnormal inputs before and after.  The projection only
+// uses min(1, rsqrt(n2)), which is 1 for every subnormal n2 and for 0 either way
+// (the same bits).  1024 x 1024 x 1000, 5 iterations: 9.42 ms instead of 9.73;
+// with the norms' square roots 1.04 instead of 1.13 ms at 1280 x 1024 x 64.
 __device__ __forceinline__ float rsqrt_approx(float x) {
   float r;
-  asm("rsqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
 
