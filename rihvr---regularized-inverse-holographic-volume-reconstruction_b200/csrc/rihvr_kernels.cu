@@ -226,13 +226,14 @@ cudaError_t launch_sum_slabs(const float2* const* src, int n, float2* dst, long 
 constexpr int RED_THREADS = 256;
 constexpr int RED_SLICES = 512;
 
-__global__ void __launch_bounds__(RED_THREADS) k_reduce_stage(const double* __restrict__ in, int n, int per_block,
-                                                              double* __restrict__ out) {
-  __shared__ double red[RED_THREADS / 32][kNumSums];
+template <int NT>
+__global__ void __launch_bounds__(NT) k_reduce_stage(const double* __restrict__ in, int n, int per_block,
+                                                     double* __restrict__ out) {
+  __shared__ double red[NT / 32][kNumSums];
   const int b0 = blockIdx.x * per_block, b1 = min(n, b0 + per_block);
   // thread j handles slot j % kNumSums of rows b0 + j / kNumSums, strided
   const int slot = threadIdx.x % kNumSums, lane_row = threadIdx.x / kNumSums;
-  constexpr int ROWS_PER_PASS = RED_THREADS / kNumSums;
+  constexpr int ROWS_PER_PASS = NT / kNumSums;
   double v = 0.0;
   for (int b = b0 + lane_row; b < b1; b += ROWS_PER_PASS) v += in[(size_t)b * kNumSums + slot];
   // gather per-slot sums: rows of the same slot are kNumSums lanes apart
@@ -243,7 +244,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_reduce_stage(const double* __re
   __syncthreads();
   if (threadIdx.x < kNumSums) {
     double s = 0.0;
-    for (int w = 0; w < RED_THREADS / 32; ++w) s += red[w][threadIdx.x];
+    for (int w = 0; w < NT / 32; ++w) s += red[w][threadIdx.x];
     out[(size_t)blockIdx.x * kNumSums + threadIdx.x] = s;
   }
 }
@@ -251,13 +252,17 @@ __global__ void __launch_bounds__(RED_THREADS) k_reduce_stage(const double* __re
 cudaError_t launch_reduce_partials(const double* partials, int nblocks, double* scratch, double* out,
                                    cudaStream_t st) {
   if (nblocks <= RED_THREADS) {
-    k_reduce_stage<<<1, RED_THREADS, 0, st>>>(partials, nblocks, nblocks, out);
+    k_reduce_stage<RED_THREADS><<<1, RED_THREADS, 0, st>>>(partials, nblocks, nblocks, out);
+    return cudaGetLastError();
+  }
+  if (nblocks <= kReduceOneLaunch) {  // 16 rows a thread at most: shorter than a second launch
+    k_reduce_stage<1024><<<1, 1024, 0, st>>>(partials, nblocks, nblocks, out);
     return cudaGetLastError();
   }
   const int per = (nblocks + RED_SLICES - 1) / RED_SLICES;
   const int slices = (nblocks + per - 1) / per;
-  k_reduce_stage<<<slices, RED_THREADS, 0, st>>>(partials, nblocks, per, scratch);
-  k_reduce_stage<<<1, RED_THREADS, 0, st>>>(scratch, slices, slices, out);
+  k_reduce_stage<RED_THREADS><<<slices, RED_THREADS, 0, st>>>(partials, nblocks, per, scratch);
+  k_reduce_stage<RED_THREADS><<<1, RED_THREADS, 0, st>>>(scratch, slices, slices, out);
   return cudaGetLastError();
 }
 

@@ -391,12 +391,22 @@ int residual_spectrum(rihvr_ctx* c) {
 
 int reduce_into(rihvr_ctx* c, int nblocks, int slot) {
   KL(launch_reduce_partials(c->partials, nblocks, c->red_scratch, c->sums_d + slot * kNumSums, c->st));
-  if (nblocks > 256) ++c->launches;  // two-stage reduction
+  if (nblocks > kReduceOneLaunch) ++c->launches;  // two-stage reduction
   return RIHVR_OK;
 }
 
-// G = A^H r: column pass from the spectrum, then the inverse row pass.
-int adjoint_volume(rihvr_ctx* c) {
+// Hologram momentum with `beta` (or its device copy), the residual at the new
+// momentum point, its squared norm into SLOT_MOM and its spectrum.
+int momentum_spectrum(rihvr_ctx* c, float beta, const float* dbeta = nullptr) {
+  int nb = 0;
+  KL(launch_holo_momentum(c->dnew, c->dY0, c->dX, c->b, c->r, beta, (long long)c->HW, c->partials, &nb, c->st, dbeta));
+  RC(reduce_into(c, nb, SLOT_MOM));
+  return residual_spectrum(c);
+}
+
+// A^H r into `out` (G unless given): column pass from the spectrum, then the
+// inverse row pass.
+int adjoint_volume(rihvr_ctx* c, float2* out = nullptr) {
   NvtxRange nvtx_("rihvr: adjoint");
   {
     ProfScope ps(c, K_ADJ_COL);
@@ -407,7 +417,7 @@ int adjoint_volume(rihvr_ctx* c) {
   }
   {
     ProfScope ps(c, K_ADJ_ROW);
-    KL(launch_rows(1, ELEM_C32, c->U, ELEM_C32, c->G, c->W, (long long)c->Nz * c->H, 1.0f, c->st));
+    KL(launch_rows(1, ELEM_C32, c->U, ELEM_C32, out ? out : c->G, c->W, (long long)c->Nz * c->H, 1.0f, c->st));
   }
   return RIHVR_OK;
 }
@@ -524,10 +534,7 @@ int state_reset(rihvr_ctx* c) {
   c->log.clear();
   c->pending_x = -1;
   // x = 0: d = 0, r = -b (:273)
-  int nb = 0;
-  KL(launch_holo_momentum(c->dnew, c->dY0, c->dX, c->b, c->r, 0.f, (long long)c->HW, c->partials, &nb, c->st));
-  RC(reduce_into(c, nb, SLOT_MOM));
-  RC(residual_spectrum(c));
+  RC(momentum_spectrum(c, 0.f));
   RC(fetch_sums(c));
   c->prev_f_resid = 0.5 * c->sums_h[SLOT_MOM * kNumSums + SUM_RR];
   return RIHVR_OK;
@@ -571,11 +578,7 @@ int enqueue_attempt(rihvr_ctx* c, bool with_adjoint) {
 // Hologram momentum, residual at the new momentum point and its spectrum.
 int enqueue_momentum(rihvr_ctx* c) {
   CK(cudaMemcpyAsync(c->scal_d + 8, c->scal_h + 8, sizeof(float), cudaMemcpyHostToDevice, c->st));
-  int nb = 0;
-  KL(launch_holo_momentum(c->dnew, c->dY0, c->dX, c->b, c->r, c->scal_h[8], (long long)c->HW, c->partials, &nb,
-                          c->st, c->scal_d + 8));
-  RC(reduce_into(c, nb, SLOT_MOM));
-  RC(residual_spectrum(c));
+  RC(momentum_spectrum(c, c->scal_h[8], c->scal_d + 8));
   CK(cudaMemcpyAsync(c->sums_h, c->sums_d, sizeof(double) * kNumSums * NUM_SLOTS, cudaMemcpyDeviceToHost, c->st));
   return RIHVR_OK;
 }
@@ -648,11 +651,7 @@ int enqueue_momentum_dev(rihvr_ctx* c) {
   KL((k_ctl_finish<<<1, 1, 0, c->st>>>(c->ctl_d, c->sums_d, c->scal_d, c->dlog_d,
                                        (double)c->p.regularization_param, tv_weight(c)),
       cudaGetLastError()));
-  int nb = 0;
-  KL(launch_holo_momentum(c->dnew, c->dY0, c->dX, c->b, c->r, 0.f, (long long)c->HW, c->partials, &nb, c->st,
-                          c->scal_d + 8));
-  RC(reduce_into(c, nb, SLOT_MOM));
-  RC(residual_spectrum(c));
+  RC(momentum_spectrum(c, 0.f, c->scal_d + 8));
   KL((k_ctl_post<<<1, 1, 0, c->st>>>(c->ctl_d, c->sums_d, c->dlog_d), cudaGetLastError()));
   return RIHVR_OK;
 }
@@ -1304,6 +1303,24 @@ int copy_out(rihvr_ctx* c, void* dst, const void* src, size_t bytes, int is_devi
 int copy_in(rihvr_ctx* c, void* dst, const void* src, size_t bytes, int is_device) {
   CK(cudaMemcpyAsync(dst, src, bytes, is_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, c->st));
   return RIHVR_OK;
+}
+
+// May the operators' row passes work on a caller's volume where it lies,
+// without a copy through the context's own (16 bytes a voxel of traffic)?  It
+// must be plain device memory of the context's device, aligned for complex
+// loads, and not overlap the intermediate volume the passes run through (which
+// rihvr_get_volume_ptr hands out).  Anything else - memory of another device,
+// managed memory, an odd address - goes through the copy.
+bool usable_in_place(const rihvr_ctx* c, const void* p) {
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (at.type != cudaMemoryTypeDevice || at.device != c->device) return false;
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p), u = reinterpret_cast<uintptr_t>(c->U);
+  const size_t bytes = sizeof(float2) * c->V;
+  return (a % sizeof(float2)) == 0 && (a + bytes <= u || u + bytes <= a);
 }
 
 int validate(const rihvr_params* p, int W, int H) {
@@ -2409,10 +2426,7 @@ int start_from_U(rihvr_ctx* c) {
   // the estimated hologram of the stored x0, then the momentum step with beta = 0:
   // d(x) = d(P_k) = A x0, r = d - b and its spectrum
   RC(forward_volume(c, elem_kind(c->storage), c->vol[c->iCur]));
-  int nb = 0;
-  KL(launch_holo_momentum(c->dnew, c->dY0, c->dX, c->b, c->r, 0.f, (long long)c->HW, c->partials, &nb, c->st));
-  RC(reduce_into(c, nb, SLOT_MOM));
-  RC(residual_spectrum(c));
+  RC(momentum_spectrum(c, 0.f));
   RC(fetch_sums(c));
   c->prev_f_resid = 0.5 * c->sums_h[SLOT_MOM * kNumSums + SUM_RR];
   return RIHVR_OK;
@@ -2577,8 +2591,12 @@ int rihvr_lipschitz(rihvr_ctx* c, int iterations, unsigned long long seed, doubl
 
 int rihvr_forward(rihvr_ctx* c, const float* volume, float* holo_out, int is_device) {
   if (!c || !volume || !holo_out) return fail(RIHVR_ERR_INVALID_ARGUMENT, "NULL argument");
-  RC(copy_in(c, c->G, volume, sizeof(float2) * c->V, is_device));
-  RC(forward_volume(c, ELEM_C32, c->G));
+  const void* src = volume;
+  if (!is_device || !usable_in_place(c, volume)) {
+    RC(copy_in(c, c->G, volume, sizeof(float2) * c->V, is_device));
+    src = c->G;
+  }
+  RC(forward_volume(c, ELEM_C32, src));
   RC(check_col_waits(c));
   return copy_out(c, holo_out, c->dnew, sizeof(float) * c->HW, is_device);
 }
@@ -2587,6 +2605,11 @@ int rihvr_adjoint(rihvr_ctx* c, const float* residual, float* volume_out, int is
   if (!c || !residual || !volume_out) return fail(RIHVR_ERR_INVALID_ARGUMENT, "NULL argument");
   RC(copy_in(c, c->r, residual, sizeof(float) * c->HW, is_device));
   RC(residual_spectrum(c));
+  if (is_device && usable_in_place(c, volume_out)) {
+    RC(adjoint_volume(c, reinterpret_cast<float2*>(volume_out)));
+    CK(cudaStreamSynchronize(c->st));
+    return RIHVR_OK;
+  }
   RC(adjoint_volume(c));
   return copy_out(c, volume_out, c->G, sizeof(float2) * c->V, is_device);
 }
