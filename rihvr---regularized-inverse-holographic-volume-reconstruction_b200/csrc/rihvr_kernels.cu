@@ -373,6 +373,101 @@ cudaError_t launch_holo_momentum(const float* dnew, float* dY0, float* dX, const
   return cudaGetLastError();
 }
 
+// A small frame's iteration is a chain of short launches, and one plane fills
+// few SMs: the two inverse and two forward passes of the hologram, its pointwise
+// steps and their reductions were ten launches and a third of an iteration at
+// 128 x 128 x 32 (38 of 118 us; 54 of 276 at 384 x 384 x 40).  These two are
+// what is left of them in the loop.
+__global__ void __launch_bounds__(FLAT_THREADS) k_spec_residual(const float2* __restrict__ parts, int nparts,
+                                                                const float2* __restrict__ Bh,
+                                                                float2* __restrict__ Dn, int W, int H, SpecSums s) {
+  const size_t HW = (size_t)W * H;
+  const unsigned half = (unsigned)(H / 2 + 1) * (unsigned)W;  // H is even
+  double acc = 0.0;
+  for (unsigned i = blockIdx.x * FLAT_THREADS + threadIdx.x; i < half; i += gridDim.x * FLAT_THREADS) {
+    const unsigned y = i / (unsigned)W, x = i - y * (unsigned)W;
+    const unsigned p = (y ? H - y : 0) * (unsigned)W + (x ? W - x : 0);  // the element at -f
+    float2 a = parts[i], b = parts[p];
+    for (int k = 1; k < nparts; ++k) {
+      a = cadd(a, parts[k * HW + i]);
+      b = cadd(b, parts[k * HW + p]);
+    }
+    const float2 d = make_float2(0.5f * (a.x + b.x), 0.5f * (a.y - b.y));
+    const bool pair = y > 0 && y < (unsigned)H / 2;  // else the partner's own thread writes it
+    Dn[i] = d;
+    if (pair) Dn[p] = make_float2(d.x, -d.y);
+    if (Bh) {
+      const float2 e = csub(d, Bh[i]);
+      const double q = (double)e.x * (double)e.x + (double)e.y * (double)e.y;
+      acc += pair ? 2.0 * q : q;
+    }
+  }
+  if (Bh) last_block_rr<FLAT_THREADS>(acc / (double)HW, s.partials, s.sums, s.counter);
+}
+
+cudaError_t launch_spec_residual(const float2* parts, int nparts, const float2* Bh, float2* Dn, int W, int H,
+                                 const SpecSums& s, cudaStream_t st) {
+  k_spec_residual<<<flat_blocks((size_t)(H / 2 + 1) * W), FLAT_THREADS, 0, st>>>(parts, nparts, Bh, Dn, W, H, s);
+  return cudaGetLastError();
+}
+
+__global__ void __launch_bounds__(FLAT_THREADS) k_spec_momentum(const float2* __restrict__ Dn, float2* D0,
+                                                                float2* __restrict__ DX,
+                                                                const float2* __restrict__ Bh,
+                                                                float2* __restrict__ Rs, float beta0,
+                                                                const float* __restrict__ dbeta, long long n,
+                                                                float scale, SpecSums s) {
+  const float beta = dbeta ? __ldg(dbeta) : beta0;  // device copy for captured launches
+  double acc = 0.0;
+  for (long long i = (long long)blockIdx.x * FLAT_THREADS + threadIdx.x; i < n; i += (long long)gridDim.x * FLAT_THREADS) {
+    const float2 d = Dn[i], d0 = D0[i];
+    const float2 x = make_float2(fmaf(beta, d.x - d0.x, d.x), fmaf(beta, d.y - d0.y, d.y));
+    DX[i] = x;
+    D0[i] = d;
+    const float2 e = csub(x, Bh[i]);
+    Rs[i] = cscale(e, scale);
+    acc += (double)e.x * (double)e.x + (double)e.y * (double)e.y;
+  }
+  last_block_rr<FLAT_THREADS>(acc / (double)n, s.partials, s.sums, s.counter);
+}
+
+cudaError_t launch_spec_momentum(const float2* Dn, float2* D0, float2* DX, const float2* Bh, float2* Rs, float beta,
+                                 const float* dbeta, long long n, const SpecSums& s, cudaStream_t st) {
+  k_spec_momentum<<<flat_blocks((size_t)n), FLAT_THREADS, 0, st>>>(Dn, D0, DX, Bh, Rs, beta, dbeta, n,
+                                                                  1.0f / (float)n, s);
+  return cudaGetLastError();
+}
+
+__global__ void k_spec_pair(const float2* __restrict__ D0, const float2* __restrict__ DX, float2* __restrict__ out,
+                            long long n) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const float2 a = D0[i], b = DX[i];
+    out[i] = make_float2(a.x - b.y, a.y + b.x);
+  }
+}
+
+cudaError_t launch_spec_pair(const float2* D0, const float2* DX, float2* out, long long n, cudaStream_t st) {
+  k_spec_pair<<<flat_blocks((size_t)n), FLAT_THREADS, 0, st>>>(D0, DX, out, n);
+  return cudaGetLastError();
+}
+
+__global__ void k_spec_fields(const float2* __restrict__ in, const float* __restrict__ b, float* __restrict__ d0,
+                              float* __restrict__ d1, float* __restrict__ dX, float* __restrict__ r, long long n) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const float2 v = in[i];
+    d0[i] = v.x;
+    d1[i] = v.x;
+    dX[i] = v.y;
+    r[i] = v.y - b[i];
+  }
+}
+
+cudaError_t launch_spec_fields(const float2* in, const float* b, float* d0, float* d1, float* dX, float* r, long long n,
+                               cudaStream_t st) {
+  k_spec_fields<<<flat_blocks((size_t)n), FLAT_THREADS, 0, st>>>(in, b, d0, d1, dX, r, n);
+  return cudaGetLastError();
+}
+
 // L1 and TV norms of the momentum point x = P + beta (P - Pprev):
 // calcL1NormComplex (sparse_volume.cu:194-235), calcTVNorm2d (:365-446),
 // calcTVNorm (:240-363, periodic in z).

@@ -124,6 +124,28 @@ cudaError_t launch_finish_forward(const float2* c, const float* b, float* dnew, 
 cudaError_t launch_holo_momentum(const float* dnew, float* dY0, float* dX, const float* b, float* r,
                                  float beta, long long n, double* partials, int* nblocks_out, cudaStream_t st,
                                  const float* dbeta = nullptr);
+// The hologram's part of an iteration in the frequency domain.  The estimated
+// hologram d = Re(IFFT2(S)) / (W H) has the spectrum (S(f) + conj S(-f)) / 2,
+// the momentum in hologram space is linear, and sum r^2 is sum |R|^2 / (W H),
+// so neither the residual's norm nor its spectrum needs a transform.
+// SpecSums: where the sum of squares goes (one double a block of partials, the
+// kNumSums sums that receive SUM_RR, a block counter that is 0 between launches).
+struct SpecSums {
+  double* partials;
+  double* sums;
+  unsigned* counter;
+};
+// Dn = Hermitian part of the sum of `nparts` spectra; with Bh, sum |Dn - Bh|^2 / (W H)
+cudaError_t launch_spec_residual(const float2* parts, int nparts, const float2* Bh, float2* Dn, int W, int H,
+                                 const SpecSums& s, cudaStream_t st);
+// DX = Dn + beta (Dn - D0), D0 = Dn, Rs = (DX - Bh) / (W H), sum |DX - Bh|^2 / (W H)
+cudaError_t launch_spec_momentum(const float2* Dn, float2* D0, float2* DX, const float2* Bh, float2* Rs, float beta,
+                                 const float* dbeta, long long n, const SpecSums& s, cudaStream_t st);
+// Two Hermitian spectra as one (out = D0 + i DX), and after its inverse
+// transform their real fields: d0 = d1 = Re, dX = Im, r = dX - b
+cudaError_t launch_spec_pair(const float2* D0, const float2* DX, float2* out, long long n, cudaStream_t st);
+cudaError_t launch_spec_fields(const float2* in, const float* b, float* d0, float* d1, float* dX, float* r, long long n,
+                               cudaStream_t st);
 cudaError_t launch_momentum_norms(int storage, const void* P, const void* Pprev, float beta, int W, int H,
                                   int Nz, int mode, double* partials, int* nblocks_out, cudaStream_t st);
 cudaError_t launch_materialize_x(int storage, const void* P, const void* Pprev, float beta, float2* out,

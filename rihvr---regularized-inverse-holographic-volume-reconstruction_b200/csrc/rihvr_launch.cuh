@@ -63,6 +63,43 @@ __device__ __forceinline__ void block_write_sums(double (&acc)[kNumSums], double
   }
 }
 
+// A sum finished by the block that ends last: partials[block] = this block's
+// sum; the last one to arrive adds them up in a fixed order into
+// sums[SUM_RR] (the other sums of the slot become 0) and leaves the counter at
+// 0 for the next launch.  Saves the one or two reduction launches that would
+// follow a small kernel.  No block waits for another.
+template <int NT>
+__device__ __forceinline__ void last_block_rr(double acc, double* partials, double* sums, unsigned* counter) {
+  __shared__ double red[NT / 32];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  double v = warp_sum(acc);
+  if (lane == 0) red[wid] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0;
+    for (int w = 0; w < NT / 32; ++w) s += red[w];
+    partials[blockIdx.x] = s;
+    __threadfence();
+    last = atomicInc(counter, gridDim.x - 1) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double t = 0;
+  for (unsigned b = threadIdx.x; b < gridDim.x; b += NT) t += __ldcg(partials + b);
+  t = warp_sum(t);
+  __syncthreads();
+  if (lane == 0) red[wid] = t;
+  __syncthreads();
+  if (threadIdx.x < kNumSums) {
+    double s = 0;
+    if (threadIdx.x == SUM_RR)
+      for (int w = 0; w < NT / 32; ++w) s += red[w];
+    sums[threadIdx.x] = s;
+  }
+}
+
 // Restart statistic weights: sparse_fistaRestart_kernel<512> (RIHVR
 // sparse_compressive_holo.cu:4393-4432) overwrites the second element's real
 // product with its imaginary one and re-adds the first element's imaginary

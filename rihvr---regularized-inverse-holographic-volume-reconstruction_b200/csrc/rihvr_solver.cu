@@ -202,6 +202,10 @@ struct rihvr_ctx {
   float2* pc1 = nullptr;
   float2* pc2 = nullptr;
   float2* Rs = nullptr;   // residual spectrum / (W H)
+  // the hologram's side of the iteration in the frequency domain: spectra of b,
+  // of the estimates of P_{k+1} and P_k, and of the momentum point
+  float2 *Bh = nullptr, *Dn = nullptr, *D0 = nullptr, *DX = nullptr;
+  unsigned* block_count = nullptr;  // of the kernels that finish their own sums: 0 between launches
   float* b = nullptr;
   float* dnew = nullptr;
   float* dY0 = nullptr;
@@ -395,13 +399,38 @@ int reduce_into(rihvr_ctx* c, int nblocks, int slot) {
   return RIHVR_OK;
 }
 
-// Hologram momentum with `beta` (or its device copy), the residual at the new
-// momentum point, its squared norm into SLOT_MOM and its spectrum.
+SpecSums spec_sums(const rihvr_ctx* c, int slot) {
+  return SpecSums{c->partials, c->sums_d + slot * kNumSums, c->block_count};
+}
+
+// dst = spectrum of the real plane src (exactly Hermitian)
+int plane_spectrum(rihvr_ctx* c, const float* src, float2* dst) {
+  ProfScope ps(c, K_PLANE);
+  KL(launch_rows(0, ELEM_R32, src, ELEM_C32, c->pc1, c->W, c->H, 1.0f, c->st));
+  KL(launch_plane_col(0, c->pc1, c->pc2, c->W, c->H, 1.0f, c->st));
+  KL(launch_spec_residual(c->pc2, 1, nullptr, dst, c->W, c->H, spec_sums(c, SLOT_FWD), c->st));
+  return RIHVR_OK;
+}
+
+// Hologram momentum with `beta` (or its device copy), the residual's spectrum
+// at the new momentum point and its squared norm into SLOT_MOM.
 int momentum_spectrum(rihvr_ctx* c, float beta, const float* dbeta = nullptr) {
-  int nb = 0;
-  KL(launch_holo_momentum(c->dnew, c->dY0, c->dX, c->b, c->r, beta, (long long)c->HW, c->partials, &nb, c->st, dbeta));
-  RC(reduce_into(c, nb, SLOT_MOM));
-  return residual_spectrum(c);
+  ProfScope ps(c, K_PLANE);
+  KL(launch_spec_momentum(c->Dn, c->D0, c->DX, c->Bh, c->Rs, beta, dbeta, (long long)c->HW, spec_sums(c, SLOT_MOM),
+                          c->st));
+  return RIHVR_OK;
+}
+
+// The holograms after a run of iterations, from their spectra: d of the last
+// prox output (dnew = dY0), d of the momentum point (dX) and its residual, two
+// real fields in one complex inverse transform.
+int spatial_holograms(rihvr_ctx* c) {
+  ProfScope ps(c, K_PLANE);
+  KL(launch_spec_pair(c->D0, c->DX, c->pc2, (long long)c->HW, c->st));
+  KL(launch_plane_col(1, c->pc2, c->pc1, c->W, c->H, 1.0f, c->st));
+  KL(launch_rows(1, ELEM_C32, c->pc1, ELEM_C32, c->pc2, c->W, c->H, 1.0f / (float)c->HW, c->st));
+  KL(launch_spec_fields(c->pc2, c->b, c->dnew, c->dY0, c->dX, c->r, (long long)c->HW, c->st));
+  return RIHVR_OK;
 }
 
 // A^H r into `out` (G unless given): column pass from the spectrum, then the
@@ -422,9 +451,9 @@ int adjoint_volume(rihvr_ctx* c, float2* out = nullptr) {
   return RIHVR_OK;
 }
 
-// S = sum over the context's planes of H'_z FFT2(vol_z) (the volume in `kind`
-// layout): the row and column passes and the sum of the z-chunks.
-int forward_partial(rihvr_ctx* c, int kind, const void* vol) {
+// The z-chunks' sums over the context's planes of H'_z FFT2(vol_z) into Spart
+// (the volume in `kind` layout): the row and column passes.
+int forward_chunks(rihvr_ctx* c, int kind, const void* vol) {
   {
     ProfScope ps(c, K_FWD_ROW);
     KL(launch_rows(0, kind, vol, ELEM_C32, c->U, c->W, (long long)c->Nz * c->H, 1.0f, c->st));
@@ -436,6 +465,12 @@ int forward_partial(rihvr_ctx* c, int kind, const void* vol) {
     KL(launch_fwd_col(c->U, c->cturn, c->zlist, c->Spart, c->W, c->H, 0, c->Nz, c->nchunks, c->st,
                       hor ? c->dz_uniform : 0.0, hor));
   }
+  return RIHVR_OK;
+}
+
+// S = their sum.
+int forward_partial(rihvr_ctx* c, int kind, const void* vol) {
+  RC(forward_chunks(c, kind, vol));
   ProfScope ps(c, K_PLANE);
   KL(launch_sum_chunks(c->Spart, c->nchunks, c->S, (long long)c->HW, c->st));
   return RIHVR_OK;
@@ -449,6 +484,21 @@ int forward_from_spectrum(rihvr_ctx* c, const float2* S_all) {
   int nb = 0;
   KL(launch_finish_forward(c->pc2, c->b, c->dnew, (long long)c->HW, c->partials, &nb, c->st));
   return reduce_into(c, nb, SLOT_FWD);
+}
+
+// Spectrum of the estimated hologram (Dn) from `nparts` spectra that add up to
+// S, and its squared residual into SLOT_FWD.
+int residual_from_spectrum(rihvr_ctx* c, const float2* parts, int nparts) {
+  ProfScope ps(c, K_PLANE);
+  KL(launch_spec_residual(parts, nparts, c->Bh, c->Dn, c->W, c->H, spec_sums(c, SLOT_FWD), c->st));
+  return RIHVR_OK;
+}
+
+// The forward operator of an iteration at the stored volume vol: Dn and the squared residual.
+int forward_iterate(rihvr_ctx* c, const void* vol) {
+  NvtxRange nvtx_("rihvr: forward");
+  RC(forward_chunks(c, elem_kind(c->storage), vol));
+  return residual_from_spectrum(c, c->Spart, c->nchunks);
 }
 
 // dnew = A vol (the volume in `kind` layout), sum (dnew - b)^2 into SLOT_FWD.
@@ -534,7 +584,11 @@ int state_reset(rihvr_ctx* c) {
   c->log.clear();
   c->pending_x = -1;
   // x = 0: d = 0, r = -b (:273)
+  RC(plane_spectrum(c, c->b, c->Bh));
+  for (float2* q : {c->Dn, c->D0}) CK(cudaMemsetAsync(q, 0, sizeof(float2) * c->HW, c->st));
   RC(momentum_spectrum(c, 0.f));
+  int nb = 0;
+  KL(launch_holo_momentum(c->dnew, c->dY0, c->dX, c->b, c->r, 0.f, (long long)c->HW, c->partials, &nb, c->st));
   RC(fetch_sums(c));
   c->prev_f_resid = 0.5 * c->sums_h[SLOT_MOM * kNumSums + SUM_RR];
   return RIHVR_OK;
@@ -570,7 +624,7 @@ int enqueue_attempt(rihvr_ctx* c, bool with_adjoint) {
   CK(cudaMemcpyAsync(c->scal_d, c->scal_h, 5 * sizeof(float), cudaMemcpyHostToDevice, c->st));
   if (with_adjoint) RC(adjoint_volume(c));
   RC(prox_volume(c, c->t, true));
-  RC(forward_volume(c, elem_kind(c->storage), c->vol[c->iNew]));
+  RC(forward_iterate(c, c->vol[c->iNew]));
   CK(cudaMemcpyAsync(c->sums_h, c->sums_d, sizeof(double) * kNumSums * NUM_SLOTS, cudaMemcpyDeviceToHost, c->st));
   return RIHVR_OK;
 }
@@ -639,7 +693,7 @@ int enqueue_attempt_dev(rihvr_ctx* c, bool first, cudaGraphConditionalHandle h) 
   KL((k_ctl_prep<<<1, 1, 0, c->st>>>(c->ctl_d, c->scal_d, tv, l1, zero_thr, first ? 1 : 0), cudaGetLastError()));
   if (first) RC(adjoint_volume(c));
   RC(prox_volume(c, c->t, true));
-  RC(forward_volume(c, elem_kind(c->storage), c->vol[c->iNew]));
+  RC(forward_iterate(c, c->vol[c->iNew]));
   KL((k_ctl_decide<<<1, 1, 0, c->st>>>(c->ctl_d, c->sums_d, c->p.max_backtracks, h, c->dlog_d, first ? 1 : 0),
       cudaGetLastError()));
   return RIHVR_OK;
@@ -1291,6 +1345,7 @@ int run_iterations(rihvr_ctx* c, int n) {
   int i = 0;
   RC(eager_start(c, n, &i));
   RC(run_iterations_from(c, i, n));
+  if (n > 0) RC(spatial_holograms(c));
   return check_col_waits(c);
 }
 
@@ -1451,6 +1506,9 @@ int create_ctx(const rihvr_params* params, int width, int height, int z_first, i
   if (rc == RIHVR_OK) rc = dalloc_t(c, &c->pc1, c->HW);
   if (rc == RIHVR_OK) rc = dalloc_t(c, &c->pc2, c->HW);
   if (rc == RIHVR_OK) rc = dalloc_t(c, &c->Rs, c->HW);
+  for (float2** q : {&c->Bh, &c->Dn, &c->D0, &c->DX})
+    if (rc == RIHVR_OK) rc = dalloc_t(c, q, c->HW);
+  if (rc == RIHVR_OK) rc = dalloc_t(c, &c->block_count, 1);
   if (rc == RIHVR_OK) rc = dalloc_t(c, &c->b, c->HW);
   if (rc == RIHVR_OK) rc = dalloc_t(c, &c->dnew, c->HW);
   if (rc == RIHVR_OK) rc = dalloc_t(c, &c->dY0, c->HW);
@@ -1492,6 +1550,7 @@ int create_ctx(const rihvr_params* params, int width, int height, int z_first, i
   if (c->dz_uniform != 0) c->tune_adj_rec = adj_col_builtin(width, height, c->Nz);
   if (cudaMemcpy(c->cturn, ct.data(), sizeof(double) * ct.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(c->zlist, zl.data(), sizeof(double) * zl.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaMemsetAsync(c->block_count, 0, sizeof(unsigned), c->st) != cudaSuccess ||
       cudaMemsetAsync(c->b, 0, sizeof(float) * c->HW, c->st) != cudaSuccess)
     return cleanup(fail(RIHVR_ERR_CUDA, "initial copies failed"));
   *out = c;
@@ -1804,7 +1863,7 @@ struct StateHeader {
 void state_header_of(const rihvr_ctx* c, StateHeader* h) {
   std::memset(h, 0, sizeof(*h));
   std::memcpy(h->magic, kStateMagic, 8);
-  h->version = 2;
+  h->version = 3;
   h->W = c->W;
   h->H = c->H;
   h->Nz = c->Nz;
@@ -1862,9 +1921,10 @@ int state_read_dev(rihvr_ctx* c, FILE* f, void* dev, size_t bytes, void* stage) 
   return RIHVR_OK;
 }
 
-// the buffers a checkpoint carries, in file order
+// the buffers a checkpoint carries, in file order (version 2 files end before
+// the spectrum of the last prox output's hologram)
 template <typename F>
-int each_state_buffer(rihvr_ctx* c, F fn) {
+int each_state_buffer(rihvr_ctx* c, int version, F fn) {
   const size_t HW = c->HW;
   RC(fn(c->b, sizeof(float) * HW));
   RC(fn(c->dnew, sizeof(float) * HW));
@@ -1873,7 +1933,8 @@ int each_state_buffer(rihvr_ctx* c, F fn) {
   RC(fn(c->r, sizeof(float) * HW));
   RC(fn(c->Rs, sizeof(float2) * HW));
   RC(fn(c->vol[c->iCur], c->esize * c->V));
-  return fn(c->vol[c->iPrev], c->esize * c->V);
+  RC(fn(c->vol[c->iPrev], c->esize * c->V));
+  return version >= 3 ? fn(c->D0, sizeof(float2) * HW) : RIHVR_OK;
 }
 
 }  // namespace
@@ -1901,7 +1962,7 @@ int rihvr_save_state(rihvr_ctx* c, const char* path) {
   PinnedGuard stage;
   CK(cudaMallocHost(&stage.p, kStateChunk));
   CK(cudaStreamSynchronize(c->st));
-  RC(each_state_buffer(c, [&](const void* dev, size_t bytes) { return state_write_dev(c, fg.f, dev, bytes, stage.p); }));
+  RC(each_state_buffer(c, h.version, [&](const void* dev, size_t bytes) { return state_write_dev(c, fg.f, dev, bytes, stage.p); }));
   if (std::fflush(fg.f) != 0) return fail(RIHVR_ERR_BAD_FILENAME, "writing the state file failed");
   return RIHVR_OK;
 }
@@ -1912,7 +1973,8 @@ int rihvr_load_state(rihvr_ctx* c, const char* path) {
   fg.f = std::fopen(path, "rb");
   if (!fg.f) return fail(RIHVR_ERR_BAD_FILENAME, std::string("cannot open ") + path);
   StateHeader h, mine;
-  if (std::fread(&h, sizeof(h), 1, fg.f) != 1 || std::memcmp(h.magic, kStateMagic, 8) != 0 || h.version != 2)
+  if (std::fread(&h, sizeof(h), 1, fg.f) != 1 || std::memcmp(h.magic, kStateMagic, 8) != 0 || h.version < 2 ||
+      h.version > 3)
     return fail(RIHVR_ERR_INVALID_FILE, "not a reconstruction state file");
   state_header_of(c, &mine);
   // the solve it resumes must be this context's: sizes, storage, mode and the
@@ -1934,8 +1996,10 @@ int rihvr_load_state(rihvr_ctx* c, const char* path) {
   c->iPrev = 0;
   c->iCur = 1;
   c->iNew = 2;
-  const int rc =
-      each_state_buffer(c, [&](void* dev, size_t bytes) { return state_read_dev(c, fg.f, dev, bytes, stage.p); });
+  int rc =
+      each_state_buffer(c, h.version, [&](void* dev, size_t bytes) { return state_read_dev(c, fg.f, dev, bytes, stage.p); });
+  if (rc == RIHVR_OK) rc = plane_spectrum(c, c->b, c->Bh);
+  if (rc == RIHVR_OK && h.version < 3) rc = plane_spectrum(c, c->dY0, c->D0);
   if (rc != RIHVR_OK) {
     c->have_holo = false;  // partly overwritten: the context needs a hologram again
     return rc;
@@ -2094,7 +2158,7 @@ int slab_attempt(const SlabGroup& g, bool first, double* sp, double* f_resid) {
   for (int i = 0; i < g.n; ++i) {
     rihvr_ctx* c = g.cs[i];
     DeviceScope ds(c->device);
-    RC(forward_from_spectrum(c, total[(size_t)i]));
+    RC(residual_from_spectrum(c, total[(size_t)i], 1));
     CK(cudaMemcpyAsync(c->sums_h, c->sums_d, sizeof(double) * kNumSums * NUM_SLOTS, cudaMemcpyDeviceToHost, c->st));
   }
   for (int i = 0; i < g.n; ++i) {
@@ -2216,6 +2280,7 @@ int rihvr_slab_iterate(rihvr_ctx* const* ctxs, int n, int iterations, const rihv
   RC(slab_settle_pending(g));
   for (int i = 0; i < n; ++i) {
     DeviceScope ds(ctxs[i]->device);
+    if (iterations > 0) RC(spatial_holograms(ctxs[i]));
     RC(check_col_waits(ctxs[i]));
   }
   return RIHVR_OK;
@@ -2345,6 +2410,7 @@ int rihvr_reconstruct_batch(rihvr_ctx* const* ctxs, int n, const float* const* h
   each_frame([&](int i, rihvr_ctx* c) -> int {
     if (combined) RC(settle_pending(c));
     else RC(run_iterations_from(c, ran[i], c->p.num_inverse_iterations));
+    if (c->p.num_inverse_iterations > 0) RC(spatial_holograms(c));
     double f = 0.0;
     RC(rihvr_objective(c, &f, nullptr));
     if (final_objectives) final_objectives[i] = f;
@@ -2425,8 +2491,9 @@ int start_from_U(rihvr_ctx* c) {
   CK(cudaMemcpyAsync(c->vol[c->iPrev], c->vol[c->iCur], c->esize * c->V, cudaMemcpyDeviceToDevice, c->st));
   // the estimated hologram of the stored x0, then the momentum step with beta = 0:
   // d(x) = d(P_k) = A x0, r = d - b and its spectrum
-  RC(forward_volume(c, elem_kind(c->storage), c->vol[c->iCur]));
+  RC(forward_iterate(c, c->vol[c->iCur]));
   RC(momentum_spectrum(c, 0.f));
+  RC(spatial_holograms(c));
   RC(fetch_sums(c));
   c->prev_f_resid = 0.5 * c->sums_h[SLOT_MOM * kNumSums + SUM_RR];
   return RIHVR_OK;
