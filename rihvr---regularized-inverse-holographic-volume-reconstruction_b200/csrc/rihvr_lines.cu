@@ -12,11 +12,11 @@
 // inputs of all its butterflies into registers (up to E elements) before a
 // barrier and writes the outputs after it.
 //
-// What bounds it: instruction issue (90 instructions an element: butterflies,
-// twiddles, index arithmetic).  Radix-4/2/3/5/7 stages between two
-// shared-memory buffers, with an index division and a table load for every
-// twiddle, took five stages at n = 1280: 883 us for a row pass of 1280 x 1024
-// x 64 on a B200, 508 us here (200 us at the memory's rate).
+// What bounds it: instruction issue (butterflies, twiddles and index arithmetic;
+// barriers and shared-memory latency keep issue near 40 %).  Radix-4/2/3/5/7
+// stages between two shared-memory buffers, with an index division and a table
+// load for every twiddle, took five stages at n = 1280: 883 us for a row pass of
+// 1280 x 1024 x 64 on a B200, 407 us here (200 us at the memory's rate).
 #include <algorithm>
 #include <cstring>
 #include <map>
@@ -36,12 +36,13 @@ constexpr int kMaxSide = 4096;
 constexpr int kMaxStages = 6;
 constexpr int kElems = 16;             // elements a thread holds at a time
 constexpr int kRowThreadsMax = 256, kColThreadsMax = 512;
-constexpr int kRowElems = 3072;        // elements of a row block's lines
+constexpr int kRowElems = 1536;        // elements of a row block's lines (blocks of 3 to 4 warps, five an SM)
 constexpr int kRowLinesMax = 128, kColsMax = 16;
 
 // one stage of radix r: m = n / r butterflies a line, ns the product of the radices before it
 struct LStage {
   int r, m, ns, tstep;         // tstep = n / (ns r): twiddle exponent of one step of k
+  int m_over_ns;               // m / ns of the second stage
   unsigned magic_m, magic_ns;  // ceil(2^32 / d): b / d = umulhi(b, magic) for b d < 2^32
 };
 struct LPlan {
@@ -89,6 +90,7 @@ bool plan_make(int n, LPlan* p) {
     s.m = n / s.r;
     s.ns = ns;
     s.tstep = n / (ns * s.r);
+    s.m_over_ns = s.m / ns;
     s.magic_m = magic(s.m);
     s.magic_ns = magic(ns);
     ns *= s.r;
@@ -105,6 +107,9 @@ int plan_threads(const LPlan& p, int lines, int e) {
   }
   return (t + 31) / 32 * 32;
 }
+
+// places a line takes in the shared copy
+int line_places(const LPlan& p) { return std::max(p.n, p.s[0].r * (p.s[0].m | 1)); }
 
 int ilog2(int c) {
   int l = 0;
@@ -129,10 +134,15 @@ int col_lines(const LPlan& p) {
   return c;
 }
 
-// A row line in shared memory gets one element of padding every 16, so that
-// the first stage's outputs (R elements apart between lanes) spread over the
-// banks; columns lie [element][column] without padding.
-__host__ __device__ __forceinline__ int padded(int i) { return i + (i >> 4); }
+// Places of a line's elements in the shared copy.  The first stage stores its
+// output r of butterfly j at r P + j, P = n / R_0 padded to an odd number, so
+// that lanes (consecutive j) write consecutive places; the second stage reads
+// element i of the sorted order at (i % R_0) P + i / R_0, which for its inputs
+// j + r m is linear in r too (R_0 divides m).  From the second stage on the
+// outputs lie in sorted order.  Every access of a butterfly is then a base and
+// a stride.  (Sorted places with one element of padding every 16 took an add
+// and a shift more for every access.)
+__host__ __device__ __forceinline__ int first_pitch(int m0) { return m0 | 1; }
 
 // w^(k r), r = 1 .. R - 1, times the inputs: w^(k r) from the table for r <= 3
 // and r = 4, 8, 12, the others as one product of two of these
@@ -167,13 +177,14 @@ __device__ __forceinline__ void twiddle_inputs(float2 (&v)[R], const float2* __r
 // One stage of radix R over the block's lines, in two halves around the
 // barrier that ends the reads of the shared copy.  split(b, m, magic_m, &c,
 // &j): line c and butterfly j of butterfly number b; load(c, i): element i of
-// line c; store(c, i, value): output element i of line c.  A thread takes
-// butterflies threadIdx.x, + blockDim.x, ...; v holds their inputs one after
-// another.  G > 0: loads or stores that carry the transfer function go in
-// groups of that many, so that the FP64 phases of all of them are not live at
-// once.
+// line c of the global input; store(q, c, i, value): its output element.  A
+// thread takes butterflies threadIdx.x, + blockDim.x, ...; v holds their
+// inputs one after another.  G > 0: loads or stores that carry the transfer
+// function go in groups of that many, so that the FP64 phases of all of them
+// are not live at once.  The shared forms get the pointer of line c's element
+// 0 from at(c) and the elements' pitch (1, or the columns of a block).
 template <int R, int E, int G, typename Split, typename Load>
-__device__ __forceinline__ void stage_load(const LStage& s, int lines, Split split, Load load, float2 (&v)[E]) {
+__device__ __forceinline__ void stage_load_global(const LStage& s, int lines, Split split, Load load, float2 (&v)[E]) {
 #pragma unroll
   for (int nb = 0; nb < butterflies(R, E); ++nb) {
     const int b = (int)threadIdx.x + nb * (int)blockDim.x;
@@ -189,27 +200,88 @@ __device__ __forceinline__ void stage_load(const LStage& s, int lines, Split spl
   }
 }
 
-template <int R, int E, int G, bool INV, bool FIRST, typename Split, typename Store>
-__device__ __forceinline__ void stage_store(const LStage& s, int lines, const float2* __restrict__ tw, Split split,
-                                            Store store, float2 (&v)[E]) {
+// SECOND: the input lies as the first stage (radix r0, pitch p0) stored it
+template <int R, int E, typename Split, typename At>
+__device__ __forceinline__ void stage_load_shared(const LStage& s, int lines, bool second, int p0, Split split, At at,
+                                                  int logp, float2 (&v)[E]) {
 #pragma unroll
   for (int nb = 0; nb < butterflies(R, E); ++nb) {
     const int b = (int)threadIdx.x + nb * (int)blockDim.x;
     if (b < s.m * lines) {
-      int c, j, k = 0;
+      int c, j, base, step;
+      split(b, s.m, s.magic_m, &c, &j);
+      if (second) {  // ns = r0: j = q r0 + k
+        const int q = (int)__umulhi((unsigned)j, s.magic_ns);
+        base = (j - q * s.ns) * p0 + q;
+        step = s.m_over_ns;
+      } else {
+        base = j;
+        step = s.m;
+      }
+      const float2* src = at(c) + ((size_t)(unsigned)base << logp);
+      step <<= logp;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        v[nb * R + r] = *src;
+        src += step;
+      }
+    }
+  }
+}
+
+// twiddles and butterflies in place: v[nb R + r] becomes output r
+template <int R, int E, bool INV, bool FIRST, typename Split>
+__device__ __forceinline__ void butterfly(const LStage& s, const float2* __restrict__ tw, int j, float2 (&a)[R], int* k) {
+  *k = 0;
+  if (!FIRST) {
+    *k = j - (int)__umulhi((unsigned)j, s.magic_ns) * s.ns;
+    twiddle_inputs<R, INV>(a, tw, *k * s.tstep);
+  }
+  reg_fft<R, INV>(a);
+}
+
+template <int R, int E, bool INV, bool FIRST, typename Split, typename At>
+__device__ __forceinline__ void stage_store_shared(const LStage& s, int lines, int p0, const float2* __restrict__ tw,
+                                                   Split split, At at, int logp, float2 (&v)[E]) {
+#pragma unroll
+  for (int nb = 0; nb < butterflies(R, E); ++nb) {
+    const int b = (int)threadIdx.x + nb * (int)blockDim.x;
+    if (b < s.m * lines) {
+      int c, j, k;
       split(b, s.m, s.magic_m, &c, &j);
       float2 a[R];
 #pragma unroll
       for (int r = 0; r < R; ++r) a[r] = v[nb * R + r];
-      if (!FIRST) {
-        k = j - (int)__umulhi((unsigned)j, s.magic_ns) * s.ns;
-        twiddle_inputs<R, INV>(a, tw, k * s.tstep);
-      }
-      reg_fft<R, INV>(a);
-      const int d = (j - k) * R + k;
+      butterfly<R, E, INV, FIRST, Split>(s, tw, j, a, &k);
+      float2* dst = at(c) + ((size_t)(unsigned)(FIRST ? j : (j - k) * R + k) << logp);
+      const int step = (FIRST ? p0 : s.ns) << logp;
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        store(nb * R + r, c, d + r * s.ns, a[r]);
+        *dst = a[r];
+        dst += step;
+      }
+    }
+  }
+}
+
+// the last stage: ns = m, so k = j and output r of butterfly j is element j + r m
+template <int R, int E, int G, bool INV, typename Split, typename Store>
+__device__ __forceinline__ void stage_store_global(const LStage& s, int lines, const float2* __restrict__ tw,
+                                                   Split split, Store store, float2 (&v)[E]) {
+#pragma unroll
+  for (int nb = 0; nb < butterflies(R, E); ++nb) {
+    const int b = (int)threadIdx.x + nb * (int)blockDim.x;
+    if (b < s.m * lines) {
+      int c, j;
+      split(b, s.m, s.magic_m, &c, &j);
+      float2 a[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) a[r] = v[nb * R + r];
+      twiddle_inputs<R, INV>(a, tw, j);  // tstep = 1
+      reg_fft<R, INV>(a);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        store(nb * R + r, c, j + r * s.m, a[r]);
         if (G > 0 && r % (G > 0 ? G : 1) == G - 1) sched_fence();
       }
     }
@@ -218,47 +290,50 @@ __device__ __forceinline__ void stage_store(const LStage& s, int lines, const fl
 
 #define RIHVR_EACH_RADIX(X) X(16) X(15) X(12) X(10) X(9) X(8) X(7) X(6) X(5) X(4) X(3) X(2)
 
-// the barrier stands outside the switches: with one in every case, the
-// compiler merged the cases around it and spilled up to 4 KB a thread
-template <int E, bool INV, bool FIRST, bool TO_SMEM, int LG, int SG, typename Split, typename Load, typename Store>
-__device__ __forceinline__ void any_stage(const LStage& s, int lines, const float2* __restrict__ tw, Split split,
-                                          Load load, Store store) {
-  float2 v[E];
-  switch (s.r) {
-#define RIHVR_CASE(RR)                                 \
-  case RR:                                             \
-    stage_load<RR, E, LG>(s, lines, split, load, v);   \
-    break;
-    RIHVR_EACH_RADIX(RIHVR_CASE)
-#undef RIHVR_CASE
-    default:
-      break;
+// one of the functions above for the stage's radix.  A barrier inside the
+// cases would make the compiler merge them around it (and spill up to 4 KB a
+// thread): the barriers stand between these switches.
+#define RIHVR_BY_RADIX(CALL)      \
+  switch (s.r) {                  \
+    RIHVR_EACH_RADIX(CALL)        \
+    default: break;               \
   }
-  if (TO_SMEM) __syncthreads();
-  switch (s.r) {
-#define RIHVR_CASE(RR)                                                \
-  case RR:                                                            \
-    stage_store<RR, E, SG, INV, FIRST>(s, lines, tw, split, store, v); \
-    break;
-    RIHVR_EACH_RADIX(RIHVR_CASE)
-#undef RIHVR_CASE
-    default:
-      break;
-  }
-  if (TO_SMEM) __syncthreads();
-}
 
 // all stages: src(c, i) the global input, dst(q, c, i, value) the global
-// output, at(c, i) an element's place in the shared copy
+// output, at(c) line c's place in the shared copy, its elements 2^logp apart
 template <int E, bool INV, int LG = 0, int SG = 0, typename Split, typename Src, typename Dst, typename At>
-__device__ __forceinline__ void line_fft(const LPlan& p, int lines, const float2* __restrict__ tw, float2* sm,
-                                         Split split, Src src, Dst dst, At at) {
-  const auto from = [=](int c, int i) { return sm[at(c, i)]; };
-  const auto to = [=](int, int c, int i, float2 v) { sm[at(c, i)] = v; };
-  any_stage<E, INV, true, true, LG, 0>(p.s[0], lines, tw, split, src, to);
+__device__ __forceinline__ void line_fft(const LPlan& p, int lines, const float2* __restrict__ tw, Split split,
+                                         Src src, Dst dst, At at, int logp) {
+  float2 v[E];
+  const int p0 = first_pitch(p.s[0].m);
+  {
+    const LStage& s = p.s[0];
+#define RIHVR_CALL(RR) case RR: stage_load_global<RR, E, LG>(s, lines, split, src, v); break;
+    RIHVR_BY_RADIX(RIHVR_CALL)
+#undef RIHVR_CALL
+    __syncthreads();
+#define RIHVR_CALL(RR) case RR: stage_store_shared<RR, E, INV, true>(s, lines, p0, tw, split, at, logp, v); break;
+    RIHVR_BY_RADIX(RIHVR_CALL)
+#undef RIHVR_CALL
+    __syncthreads();
+  }
 #pragma unroll 1
-  for (int i = 1; i + 1 < p.nst; ++i) any_stage<E, INV, false, true, 0, 0>(p.s[i], lines, tw, split, from, to);
-  any_stage<E, INV, false, false, 0, SG>(p.s[p.nst - 1], lines, tw, split, from, dst);
+  for (int i = 1; i < p.nst; ++i) {
+    const LStage& s = p.s[i];
+#define RIHVR_CALL(RR) case RR: stage_load_shared<RR, E>(s, lines, i == 1, p0, split, at, logp, v); break;
+    RIHVR_BY_RADIX(RIHVR_CALL)
+#undef RIHVR_CALL
+    if (i + 1 == p.nst) break;
+    __syncthreads();
+#define RIHVR_CALL(RR) case RR: stage_store_shared<RR, E, INV, false>(s, lines, p0, tw, split, at, logp, v); break;
+    RIHVR_BY_RADIX(RIHVR_CALL)
+#undef RIHVR_CALL
+    __syncthreads();
+  }
+  const LStage& s = p.s[p.nst - 1];
+#define RIHVR_CALL(RR) case RR: stage_store_global<RR, E, SG, INV>(s, lines, tw, split, dst, v); break;
+  RIHVR_BY_RADIX(RIHVR_CALL)
+#undef RIHVR_CALL
 }
 
 // exp(-2 pi i k / n)
@@ -318,21 +393,21 @@ bool plan_of(int n, LPlan* p) {
 template <bool INV, int IN>
 __global__ void __launch_bounds__(kRowThreadsMax, 2)
     k_line_rows(const __grid_constant__ LPlan p, const float2* __restrict__ tw, const void* __restrict__ in,
-                float2* __restrict__ out, long long nlines, float scale, int logc) {
+                float2* __restrict__ out, long long nlines, float scale, int logc, int ls) {
   extern __shared__ __align__(128) float2 gbuf[];
   const long long l0 = (long long)blockIdx.x << logc;
   const int lines = (int)min(1LL << logc, nlines - l0);
   const size_t base = (size_t)l0 * p.n;
-  const int n = p.n, ls = padded(p.n);
+  const int n = p.n;
   line_fft<kElems, INV>(
-      p, lines, tw, gbuf,
+      p, lines, tw,
       [](int b, int m, unsigned mg, int* c, int* j) {
         *c = (int)__umulhi((unsigned)b, mg);
         *j = b - *c * m;
       },
       [=](int c, int i) { return load_as<IN>(in, base + (size_t)(c * n + i)); },
       [=](int, int c, int i, float2 v) { out[base + (size_t)(c * n + i)] = cscale(v, scale); },
-      [=](int c, int i) { return c * ls + padded(i); });
+      [=](int c) { return gbuf + c * ls; }, 0);
 }
 
 template <bool INV, int IN>
@@ -341,11 +416,13 @@ cudaError_t rows_launch(const LPlan& p, const float2* tw, const void* in, float2
   const int C = row_lines(p);
   const long long blocks = (nlines + C - 1) / C;
   if (blocks <= 0) return cudaSuccess;
-  const size_t smem = sizeof(float2) * (size_t)C * padded(p.n);
+  // an odd line pitch keeps lines apart in the banks
+  const int ls = line_places(p) | 1;
+  const size_t smem = sizeof(float2) * (size_t)C * ls;
   cudaError_t e = allow_smem(k_line_rows<INV, IN>, smem);
   if (e != cudaSuccess) return e;
   k_line_rows<INV, IN>
-      <<<(unsigned)blocks, plan_threads(p, C, kElems), smem, st>>>(p, tw, in, out, nlines, scale, ilog2(C));
+      <<<(unsigned)blocks, plan_threads(p, C, kElems), smem, st>>>(p, tw, in, out, nlines, scale, ilog2(C), ls);
   return cudaGetLastError();
 }
 
@@ -360,8 +437,8 @@ struct ColSplit {
   }
 };
 struct ColAt {
-  int logc;
-  __device__ __forceinline__ int operator()(int c, int i) const { return (i << logc) + c; }
+  float2* sm;
+  __device__ __forceinline__ float2* operator()(int c) const { return sm + c; }
 };
 
 // adjoint: U_z(:, x) = IDFT_y(conj(H'_z(:, x)) Rs(:, x)), planes [zb, ze) of the block
@@ -379,7 +456,7 @@ __global__ void __launch_bounds__(kColThreadsMax, 1)
     const double zz = zlist[z];
     float2* Uz = U + (size_t)z * HW;
     line_fft<kElems, true, 4, 0>(
-        p, lines, tw, gbuf, ColSplit{logc},
+        p, lines, tw, ColSplit{logc},
         [=](int c, int y) {
           if (x0 + c >= W) return make_float2(0.f, 0.f);
           const unsigned i = (unsigned)(y * W + x0 + c);
@@ -388,7 +465,7 @@ __global__ void __launch_bounds__(kColThreadsMax, 1)
         [=](int, int c, int y, float2 v) {
           if (x0 + c < W) Uz[(unsigned)(y * W + x0 + c)] = v;
         },
-        ColAt{logc});
+        ColAt{gbuf}, logc);
   }
 }
 
@@ -399,13 +476,13 @@ __global__ void __launch_bounds__(kColThreadsMax, 1)
 __global__ void __launch_bounds__(kColThreadsMax, 1)
     k_line_fwd_col(const __grid_constant__ LPlan p, const float2* __restrict__ tw, const float2* __restrict__ T,
                    const double* __restrict__ cturn, const double* __restrict__ zlist, float2* __restrict__ Spart,
-                   int W, int z0, int z1, int zpb, int logc) {
+                   int W, int z0, int z1, int zpb, int logc, int places) {
   extern __shared__ __align__(128) float2 gbuf[];
   const int x0 = blockIdx.x << logc;
   const int lines = 1 << logc;
   const int zb = z0 + blockIdx.y * zpb, ze = min(zb + zpb, z1);
   const size_t HW = (size_t)p.n * W;
-  float2* const acc = gbuf + (p.n << logc);
+  float2* const acc = gbuf + (places << logc);
   for (int e = threadIdx.x; e < p.n << logc; e += blockDim.x) acc[e] = make_float2(0.f, 0.f);
   __syncthreads();
 #pragma unroll 1
@@ -413,7 +490,7 @@ __global__ void __launch_bounds__(kColThreadsMax, 1)
     const double zz = zlist[z];
     const float2* Tz = T + (size_t)z * HW;
     line_fft<kElems, false, 0, 4>(
-        p, lines, tw, gbuf, ColSplit{logc},
+        p, lines, tw, ColSplit{logc},
         [=](int c, int y) {
           return x0 + c < W ? __ldg(Tz + (unsigned)(y * W + x0 + c)) : make_float2(0.f, 0.f);
         },
@@ -425,7 +502,7 @@ __global__ void __launch_bounds__(kColThreadsMax, 1)
           a.y = fmaf(v.x, h.y, fmaf(v.y, h.x, a.y));
           acc[(y << logc) + c] = a;
         },
-        ColAt{logc});
+        ColAt{gbuf}, logc);
   }
   __syncthreads();
   float2* Sp = Spart + (size_t)blockIdx.y * HW;
@@ -442,12 +519,12 @@ __global__ void __launch_bounds__(kColThreadsMax, 1)
   extern __shared__ __align__(128) float2 gbuf[];
   const int x0 = blockIdx.x << logc;
   line_fft<kElems, INV>(
-      p, 1 << logc, tw, gbuf, ColSplit{logc},
+      p, 1 << logc, tw, ColSplit{logc},
       [=](int c, int y) { return x0 + c < W ? in[(unsigned)(y * W + x0 + c)] : make_float2(0.f, 0.f); },
       [=](int, int c, int y, float2 v) {
         if (x0 + c < W) out[(unsigned)(y * W + x0 + c)] = cscale(v, scale);
       },
-      ColAt{logc});
+      ColAt{gbuf}, logc);
 }
 
 // plan, table, columns a block, threads and shared memory of a column launch
@@ -466,7 +543,7 @@ cudaError_t col_launch(int W, int H, cudaStream_t st, ColLaunch* L) {
   L->logc = ilog2(L->C);
   L->strips = (W + L->C - 1) / L->C;
   L->threads = plan_threads(L->p, L->C, kElems);
-  L->smem = sizeof(float2) * (size_t)H * L->C;
+  L->smem = sizeof(float2) * (size_t)line_places(L->p) * L->C;
   return cudaSuccess;
 }
 
@@ -546,11 +623,11 @@ cudaError_t launch_line_fwd_col(const float2* T, const double* cturn, const doub
     e = cudaMemsetAsync(Spart + (size_t)chunks * H * W, 0, sizeof(float2) * (size_t)(nchunks - chunks) * H * W, st);
     if (e != cudaSuccess) return e;
   }
-  const size_t smem = 2 * L.smem;  // exchange buffer and sums
+  const size_t smem = L.smem + sizeof(float2) * (size_t)H * L.C;  // exchange buffer and sums
   e = allow_smem(k_line_fwd_col, smem);
   if (e != cudaSuccess) return e;
-  k_line_fwd_col<<<dim3(L.strips, chunks), L.threads, smem, st>>>(L.p, L.tw, T, cturn, zlist, Spart, W, z0, z1,
-                                                                    zpb, L.logc);
+  k_line_fwd_col<<<dim3(L.strips, chunks), L.threads, smem, st>>>(L.p, L.tw, T, cturn, zlist, Spart, W, z0, z1, zpb,
+                                                                  L.logc, line_places(L.p));
   return cudaGetLastError();
 }
 
