@@ -343,7 +343,10 @@ struct TvwShape {
   // bytes of spill, and 8 blocks (16 warps) share an SM; the norm terms need
   // about 160 registers, which caps them at 6 blocks (12 warps).  At
   // 1024 x 1024 x 1000 (n_tv = 5, no norm terms) a launch took 10.42 ms with
-  // 4-warp blocks at 12 warps per SM, 9.5 ms with 2-warp blocks at 16.
+  // 4-warp blocks at 12 warps per SM, 9.5 ms with 2-warp blocks at 16 (9.1 ms
+  // now).  Four columns a lane (strips of 128, a tenth fewer columns computed
+  // twice, 8 warps per SM at 221 registers, no spills) took 12.1 ms unrolled by
+  // four and 10.6 ms by two.
   static constexpr int NW = 2;
   static constexpr size_t SMEM = sizeof(float4) * (size_t)SLOT * D * NW;
   static_assert(CPL == 2 || CPL == 4, "columns per lane");
@@ -411,11 +414,12 @@ __device__ __forceinline__ void store_run(ST* p, const float2 (&v)[CPL]) {
 }
 
 template <typename ST, int NTV, bool NORMS, int CPL = 2, int NW = TvwShape<NTV, CPL>::NW,
-          int MINB = tvw_minb<NTV, NORMS>(), int UNR = 4, int PADTO = 4, int PART = 0>
+          int MINB = tvw_minb<NTV, NORMS>(), int PART = 0>
 __global__ void __launch_bounds__(32 * NW, MINB) k_prox_tv2d_strip(ProxArgs a0, TvsGrid gr) {
   const ProxArgs a = resolve_scalars(a0);
   using Sh = TvwShape<NTV, CPL>;
-  constexpr int h = Sh::h, HX = Sh::HX, VW = Sh::VW, D = Sh::D, RM = D - 1, F4 = Sh::F4;
+  constexpr int h = Sh::h, HX = Sh::HX, VW = Sh::VW, D = Sh::D, F4 = Sh::F4;
+  constexpr int UNR = 4;          // steps of an unrolled loop body
   constexpr int QS = F4 * 32;     // float4 between the arrays of a slot
   constexpr int SL = 3 * QS;      // float4 per slot
   static_assert(PART == 0 || CPL == 2, "the two-part forms move a lane's two columns as one float4");
@@ -428,9 +432,12 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_prox_tv2d_strip(ProxArgs a0, 
   const long long work = (long long)blockIdx.x * NW + w;
   const long long nwork = (long long)gr.nstrips * gr.nseg * a.Nz;
 
-  double dacc[kNumSums];
+  // the FP64 sums are touched every eighth row: in shared memory they cost no
+  // registers, which the loop is short of
+  constexpr int NS = NORMS ? kNumSums : SUM_RS + 1;  // sums this kernel accumulates
+  __shared__ double dsum[NS][32 * NW];
 #pragma unroll
-  for (int k = 0; k < kNumSums; ++k) dacc[k] = 0.0;
+  for (int k = 0; k < NS; ++k) dsum[k][threadIdx.x] = 0.0;
 
   if (work < nwork) {
     const int strip = (int)(work % gr.nstrips);
@@ -443,20 +450,19 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_prox_tv2d_strip(ProxArgs a0, 
     ST* Pn = static_cast<ST*>(a.Pnew) + plane;
     const float t = a.t, beta = a.beta;
     const float2 nmu = make_float2(-a.mu, -a.mu), s2 = make_float2(a.s, a.s);
-    const float2 bb = make_float2(beta, beta), nt2 = make_float2(-t, -t), t2 = make_float2(t, t);
+    const float2 bb = make_float2(beta, beta), nt2 = make_float2(-t, -t);
     const float2 z2 = make_float2(0.f, 0.f);
     const float thr = a.thr;
     const int faithful = a.faithful;
-    constexpr int NS = NORMS ? kNumSums : SUM_RS + 1;  // sums this kernel accumulates
 
     const int cu = strip * VW - HX + CPL * lane;   // first column of this lane, unwrapped
     const int gc = ((cu % W) + W) % W;             // a multiple of CPL; W is one too
     const bool lane_ok = (CPL * lane >= HX) && (CPL * lane < HX + VW) && (cu < W);
     const int r0 = seg * gr.seg_len;
     const int r1 = min(H, r0 + gr.seg_len);
-    // runs start up to PADTO - 1 rows earlier so that the step count is a
-    // multiple of PADTO (the unroll factor)
-    const int pad = (PADTO - ((r1 - r0 + 2 * h) % PADTO)) % PADTO;
+    // runs start up to UNR - 1 rows earlier so that the step count is a
+    // multiple of the unroll factor
+    const int pad = (UNR - ((r1 - r0 + 2 * h) % UNR)) % UNR;
     const int nsteps = (r1 - r0) + 2 * h + pad;
     // the warm-up may reach back more than one plane height on short planes
     int lrow = ((r0 - h - pad) % H + H) % H;
@@ -475,9 +481,8 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_prox_tv2d_strip(ProxArgs a0, 
       }
     };
     size_t goff = 0;  // row offset of the last main-ring request
-    auto request = [&](int slot) {
+    auto request = [&](float4* e) {
       const size_t off = (size_t)lrow * W + gc;
-      float4* e = ring + slot * SL;
       cp_async_run<ST, CPL>(e, Pp + off);
       cp_async_run<float2, CPL>(e + QS, G + off);
       cp_async_run<ST, CPL>(e + 2 * QS, P + off);
@@ -485,7 +490,7 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_prox_tv2d_strip(ProxArgs a0, 
       goff = off;
       lrow = (lrow + 1 == H) ? 0 : lrow + 1;
     };
-    request(0);
+    request(ring);
     request_g(goff, 0);
 
     float2 gX[NTV][CPL], gY[NTV][CPL], yU[NTV][CPL];
@@ -500,168 +505,193 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_prox_tv2d_strip(ProxArgs a0, 
 #pragma unroll
     for (int k = 0; k < kNumSums; ++k) acc[k] = 0.f;
 
-#pragma unroll UNR
-    for (int i = 0; i < nsteps; ++i) {
-      cp_async_wait<0>();
-      // stage 0: xh = P + beta (P - Pprev) - t G replaces Pprev in the slot
-      {
-        float4* e = ring + (i & RM) * SL;
-        float2 p[CPL], q[CPL], g[CPL];
-        ring_vals<ST, CPL>(e + 2 * QS, p);
-        ring_vals<ST, CPL>(e, q);
-        ring_vals<float2, CPL>(e + QS, g);
+    // The ring in groups of UNR slots, rotated once a loop body: the slot `back`
+    // steps behind step u of the body is a group's offset plus a constant, where
+    // a slot from the step's number took a mask and a multiply for each of the
+    // 10 or so slots a step touches (1024 x 1024 x 1000, no norms: 9.42 ms with
+    // that, 9.1 ms so, with the FP64 sums in shared memory; 1280 x 1024 x 64 with
+    // norms: 1.04 and 0.99 ms).
+    int grp[D / UNR];
 #pragma unroll
-        for (int k = 0; k < F4; ++k) {
-          const float2 xa = f2fma(nt2, g[2 * k], f2fma(bb, f2sub(p[2 * k], q[2 * k]), p[2 * k]));
-          const float2 xb = f2fma(nt2, g[2 * k + 1], f2fma(bb, f2sub(p[2 * k + 1], q[2 * k + 1]), p[2 * k + 1]));
-          e[k * 32] = make_float4(xa.x, xa.y, xb.x, xb.y);
+    for (int k = 0; k < D / UNR; ++k) grp[k] = k * UNR * SL;
+    auto slot_of = [&](int u, int back) -> float4* {
+      const int s = (u - back + 2 * D) % D;
+      return ring + grp[s / UNR] + (s % UNR) * SL;
+    };
+#pragma unroll 1
+    for (int i0 = 0; i0 < nsteps; i0 += UNR) {
+#pragma unroll
+      for (int u = 0; u < UNR; ++u) {
+        const int i = i0 + u;
+        cp_async_wait<0>();
+        // stage 0: xh = P + beta (P - Pprev) - t G replaces Pprev in the slot
+        {
+          float4* e = slot_of(u, 0);
+          float2 p[CPL], q[CPL], g[CPL];
+          ring_vals<ST, CPL>(e + 2 * QS, p);
+          ring_vals<ST, CPL>(e, q);
+          ring_vals<float2, CPL>(e + QS, g);
+#pragma unroll
+          for (int k = 0; k < F4; ++k) {
+            const float2 xa = f2fma(nt2, g[2 * k], f2fma(bb, f2sub(p[2 * k], q[2 * k]), p[2 * k]));
+            const float2 xb = f2fma(nt2, g[2 * k + 1], f2fma(bb, f2sub(p[2 * k + 1], q[2 * k + 1]), p[2 * k + 1]));
+            e[k * 32] = make_float4(xa.x, xa.y, xb.x, xb.y);
+          }
         }
-      }
-      if (i + 1 < nsteps) request((i + 1) & RM);
+        if (i + 1 < nsteps) request(slot_of(u, -1));
 
-      float2 ny[CPL];   // gy of the iteration before, on the row below
-      // iteration 1 on row j-1: g^0 = 0, so the estimate is xh itself; in the
-      // second part g^0 is the first part's dual, loaded with the rows
-      {
-        float2 y[CPL], yl[CPL], g0x[CPL], g0y[CPL];
-        ring_vals<float2, CPL>(ring + ((i - 1) & RM) * SL, y);
-        if constexpr (PART == 2) {
-          float2 g1y[CPL], gxr[CPL];
-          const float4* gp = gring + ((i - 1) & 1) * 2 * 32;  // row j-1
-          const float4* gq = gring + (i & 1) * 2 * 32;        // row j
-          ring_vals<float2, CPL>(gp, g0x);
-          ring_vals<float2, CPL>(gp + 32, g0y);
-          ring_vals<float2, CPL>(gq + 32, g1y);
+        float2 ny[CPL];   // gy of the iteration before, on the row below
+        // iteration 1 on row j-1: g^0 = 0, so the estimate is xh itself; in the
+        // second part g^0 is the first part's dual, loaded with the rows
+        {
+          float2 y[CPL], yl[CPL], g0x[CPL], g0y[CPL];
+          ring_vals<float2, CPL>(slot_of(u, 1), y);
+          if constexpr (PART == 2) {
+            float2 g1y[CPL], gxr[CPL];
+            const float4* gp = gring + ((u + 1) & 1) * 2 * 32;  // row j-1 (steps of even i0 + u at 0)
+            const float4* gq = gring + (u & 1) * 2 * 32;        // row j
+            ring_vals<float2, CPL>(gp, g0x);
+            ring_vals<float2, CPL>(gp + 32, g0y);
+            ring_vals<float2, CPL>(gq + 32, g1y);
 #pragma unroll
-          for (int c = 0; c < CPL - 1; ++c) gxr[c] = g0x[c + 1];
-          gxr[CPL - 1] = shfl_down2(g0x[0]);
+            for (int c = 0; c < CPL - 1; ++c) gxr[c] = g0x[c + 1];
+            gxr[CPL - 1] = shfl_down2(g0x[0]);
 #pragma unroll
-          for (int c = 0; c < CPL; ++c) y[c] = tv_estimate(y[c], g0x[c], gxr[c], g0y[c], g1y[c], nmu);
-          // row j-1's values have been used, so its slot is free: the next
-          // step's row goes there
-          if (i + 1 < nsteps) request_g(goff, i + 1);
-        } else {
-#pragma unroll
-          for (int c = 0; c < CPL; ++c) g0x[c] = g0y[c] = z2;
-        }
-        yl[0] = shfl_up2(y[CPL - 1]);
-#pragma unroll
-        for (int c = 1; c < CPL; ++c) yl[c] = y[c - 1];
-#pragma unroll
-        for (int c = 0; c < CPL; ++c) {
-          float2 gx = g0x[c], gy = g0y[c];
-          tv_dual(gx, gy, y[c], yl[c], yU[0][c], s2);
-          yU[0][c] = y[c];
-          ny[c] = gy;
-          // the new row replaces the one above it, which moves to (y, yl)
-          const float2 ogx = gX[0][c], ogy = gY[0][c];
-          gX[0][c] = gx;
-          gY[0][c] = gy;
-          y[c] = ogx;
-          yl[c] = ogy;
-        }
-        // from here (y, yl) carry the previous iteration's (gx, gy) on the
-        // row the next stage works on
-#pragma unroll
-        for (int L = 1; L <= NTV; ++L) {
-          // stage L+1 (iteration L+1, or the final stage when L == NTV) on row j-1-L
-          const float4* e = ring + ((i - 1 - L) & RM) * SL;
-          float2 xh[CPL];
-          ring_vals<float2, CPL>(e, xh);
-          float2 gxr[CPL], yy[CPL];
-#pragma unroll
-          for (int c = 0; c < CPL - 1; ++c) gxr[c] = y[c + 1];
-          gxr[CPL - 1] = shfl_down2(y[0]);
-#pragma unroll
-          for (int c = 0; c < CPL; ++c) yy[c] = tv_estimate(xh[c], y[c], gxr[c], yl[c], ny[c], nmu);
-          if (L < NTV) {
-            float2 yls[CPL];
-            yls[0] = shfl_up2(yy[CPL - 1]);
-#pragma unroll
-            for (int c = 1; c < CPL; ++c) yls[c] = yy[c - 1];
-#pragma unroll
-            for (int c = 0; c < CPL; ++c) {
-              float2 gx = y[c], gy = yl[c];
-              tv_dual(gx, gy, yy[c], yls[c], yU[L][c], s2);
-              yU[L][c] = yy[c];
-              ny[c] = gy;
-              const float2 ogx = gX[L][c], ogy = gY[L][c];
-              gX[L][c] = gx;
-              gY[L][c] = gy;
-              y[c] = ogx;
-              yl[c] = ogy;
-            }
-          } else if constexpr (PART == 1) {
-            // first part: (y, yl) hold this kernel's last dual on row j - h; it
-            // goes to memory for the second part instead of the estimate
-            if (i >= 2 * h + pad && lane_ok) {
-              const size_t eo = plane + (size_t)orow * W + gc;
-              *reinterpret_cast<float4*>(a.gdx + eo) = make_float4(y[0].x, y[0].y, y[1].x, y[1].y);
-              *reinterpret_cast<float4*>(a.gdy + eo) = make_float4(yl[0].x, yl[0].y, yl[1].x, yl[1].y);
-            }
+            for (int c = 0; c < CPL; ++c) y[c] = tv_estimate(y[c], g0x[c], gxr[c], g0y[c], g1y[c], nmu);
+            // row j-1's values have been used, so its slot is free: the next
+            // step's row goes there
+            if (i + 1 < nsteps) request_g(goff, i + 1);
           } else {
-            // final stage: p = shrink(estimate) on row j - h, then the sums
-            float2 p[CPL], x[CPL], g[CPL], y0[CPL];
-            ring_vals<float2, CPL>(e + QS, g);
-            ring_vals<ST, CPL>(e + 2 * QS, y0);
 #pragma unroll
-            for (int c = 0; c < CPL; ++c) {
-              p[c] = shrink(yy[c], thr, faithful);
-              x[c] = f2fma(t2, g[c], xh[c]);
-            }
-            if (i >= 2 * h + pad) {  // row orow is exact
-              float2 pl0 = z2, xl0 = z2;
-              if (NORMS) {
-                pl0 = shfl_up2(p[CPL - 1]);
-                xl0 = shfl_up2(x[CPL - 1]);
+            for (int c = 0; c < CPL; ++c) g0x[c] = g0y[c] = z2;
+          }
+          yl[0] = shfl_up2(y[CPL - 1]);
+#pragma unroll
+          for (int c = 1; c < CPL; ++c) yl[c] = y[c - 1];
+#pragma unroll
+          for (int c = 0; c < CPL; ++c) {
+            float2 gx = g0x[c], gy = g0y[c];
+            tv_dual(gx, gy, y[c], yl[c], yU[0][c], s2);
+            yU[0][c] = y[c];
+            ny[c] = gy;
+            // the new row replaces the one above it, which moves to (y, yl)
+            const float2 ogx = gX[0][c], ogy = gY[0][c];
+            gX[0][c] = gx;
+            gY[0][c] = gy;
+            y[c] = ogx;
+            yl[c] = ogy;
+          }
+          // from here (y, yl) carry the previous iteration's (gx, gy) on the
+          // row the next stage works on
+#pragma unroll
+          for (int L = 1; L <= NTV; ++L) {
+            // stage L+1 (iteration L+1, or the final stage when L == NTV) on row j-1-L
+            const float4* e = slot_of(u, 1 + L);
+            float2 xh[CPL];
+            ring_vals<float2, CPL>(e, xh);
+            float2 gxr[CPL], yy[CPL];
+#pragma unroll
+            for (int c = 0; c < CPL - 1; ++c) gxr[c] = y[c + 1];
+            gxr[CPL - 1] = shfl_down2(y[0]);
+#pragma unroll
+            for (int c = 0; c < CPL; ++c) yy[c] = tv_estimate(xh[c], y[c], gxr[c], yl[c], ny[c], nmu);
+            if (L < NTV) {
+              float2 yls[CPL];
+              yls[0] = shfl_up2(yy[CPL - 1]);
+#pragma unroll
+              for (int c = 1; c < CPL; ++c) yls[c] = yy[c - 1];
+#pragma unroll
+              for (int c = 0; c < CPL; ++c) {
+                float2 gx = y[c], gy = yl[c];
+                tv_dual(gx, gy, yy[c], yls[c], yU[L][c], s2);
+                yU[L][c] = yy[c];
+                ny[c] = gy;
+                const float2 ogx = gX[L][c], ogy = gY[L][c];
+                gX[L][c] = gx;
+                gY[L][c] = gy;
+                y[c] = ogx;
+                yl[c] = ogy;
               }
-              if (lane_ok) {
-                const size_t eo = (size_t)orow * W + gc;
-                store_run<ST, CPL>(Pn + eo, p);
-                float wr, wi;
-                restart_w(eo, faithful, &wr, &wi);
+            } else if constexpr (PART == 1) {
+              // first part: (y, yl) hold this kernel's last dual on row j - h; it
+              // goes to memory for the second part instead of the estimate
+              if (i >= 2 * h + pad && lane_ok) {
+                const size_t eo = plane + (size_t)orow * W + gc;
+                *reinterpret_cast<float4*>(a.gdx + eo) = make_float4(y[0].x, y[0].y, y[1].x, y[1].y);
+                *reinterpret_cast<float4*>(a.gdy + eo) = make_float4(yl[0].x, yl[0].y, yl[1].x, yl[1].y);
+              }
+            } else {
+              // final stage: p = shrink(estimate) on row j - h, then the sums
+              float2 p[CPL], x[CPL], g[CPL], y0[CPL];
+              ring_vals<float2, CPL>(e + QS, g);
+              ring_vals<ST, CPL>(e + 2 * QS, y0);
 #pragma unroll
-                for (int c = 0; c < CPL; ++c) {
-                  const float2 d = f2sub(p[c], x[c]);
-                  const float2 dg = f2mul(d, g[c]);
-                  acc[SUM_LIM1] += dg.x + dg.y;
-                  acc[SUM_LIM2] += cabs2(d);
-                  const float2 uv = f2mul(f2sub(x[c], p[c]), f2sub(p[c], y0[c]));
-                  acc[SUM_RS] += fmaf(wr, uv.x, wi * uv.y);
-                  if (NORMS) {
-                    const float2 pl = c ? p[c - 1] : pl0, xl = c ? x[c - 1] : xl0;
-                    acc[SUM_L1P] += norm_sqrt(cabs2(p[c]));
-                    acc[SUM_TVP] += norm_sqrt(cabs2(f2sub(pl, p[c])) + cabs2(f2sub(pu[c], p[c])));
-                    acc[SUM_L1X] += norm_sqrt(cabs2(x[c]));
-                    acc[SUM_TVX] += norm_sqrt(cabs2(f2sub(xl, x[c])) + cabs2(f2sub(xu[c], x[c])));
+              for (int c = 0; c < CPL; ++c) {
+                p[c] = shrink(yy[c], thr, faithful);
+                x[c] = make_float2(fmaf(t, g[c].x, xh[c].x), fmaf(t, g[c].y, xh[c].y));
+              }
+              if (i >= 2 * h + pad) {  // row orow is exact
+                float2 pl0 = z2, xl0 = z2;
+                if (NORMS) {
+                  pl0 = shfl_up2(p[CPL - 1]);
+                  xl0 = shfl_up2(x[CPL - 1]);
+                }
+                if (lane_ok) {
+                  const size_t eo = (size_t)orow * W + gc;
+                  store_run<ST, CPL>(Pn + eo, p);
+                  float wr, wi;
+                  restart_w(eo, faithful, &wr, &wi);
+#pragma unroll
+                  for (int c = 0; c < CPL; ++c) {
+                    const float2 d = f2sub(p[c], x[c]);
+                    acc[SUM_LIM1] = fmaf(d.x, g[c].x, fmaf(d.y, g[c].y, acc[SUM_LIM1]));
+                    acc[SUM_LIM2] = fmaf(d.x, d.x, fmaf(d.y, d.y, acc[SUM_LIM2]));
+                    const float2 dv = f2mul(d, f2sub(p[c], y0[c]));  // (x - p)(p - y0) with the sign turned
+                    acc[SUM_RS] = fmaf(-wr, dv.x, fmaf(-wi, dv.y, acc[SUM_RS]));
+                    if (NORMS) {
+                      const float2 pl = c ? p[c - 1] : pl0, xl = c ? x[c - 1] : xl0;
+                      acc[SUM_L1P] += norm_sqrt(cabs2(p[c]));
+                      acc[SUM_TVP] += norm_sqrt(cabs2(f2sub(pl, p[c])) + cabs2(f2sub(pu[c], p[c])));
+                      acc[SUM_L1X] += norm_sqrt(cabs2(x[c]));
+                      acc[SUM_TVX] += norm_sqrt(cabs2(f2sub(xl, x[c])) + cabs2(f2sub(xu[c], x[c])));
+                    }
+                  }
+                }
+                if (((i - 2 * h - pad) & 7) == 7) {  // FP32 partials over at most 8 rows
+#pragma unroll
+                  for (int k = 0; k < NS; ++k) {
+                    dsum[k][threadIdx.x] += (double)acc[k];
+                    acc[k] = 0.f;
                   }
                 }
               }
-              if (((i - 2 * h - pad) & 7) == 7) {  // FP32 partials over at most 8 rows
+              if (NORMS) {
 #pragma unroll
-                for (int k = 0; k < NS; ++k) {
-                  dacc[k] += (double)acc[k];
-                  acc[k] = 0.f;
+                for (int c = 0; c < CPL; ++c) {
+                  pu[c] = p[c];
+                  xu[c] = x[c];
                 }
-              }
-            }
-            if (NORMS) {
-#pragma unroll
-              for (int c = 0; c < CPL; ++c) {
-                pu[c] = p[c];
-                xu[c] = x[c];
               }
             }
           }
         }
+        orow = (orow + 1 == H) ? 0 : orow + 1;
       }
-      orow = (orow + 1 == H) ? 0 : orow + 1;
+      const int g0 = grp[0];
+#pragma unroll
+      for (int k = 0; k + 1 < D / UNR; ++k) grp[k] = grp[k + 1];
+      grp[D / UNR - 1] = g0;
     }
     cp_async_wait<0>();
 #pragma unroll
-    for (int k = 0; k < NS; ++k) dacc[k] += (double)acc[k];
+    for (int k = 0; k < NS; ++k) dsum[k][threadIdx.x] += (double)acc[k];
   }
-  if constexpr (PART != 1) block_write_sums<32 * NW>(dacc, a.partials, blockIdx.x);
+  if constexpr (PART != 1) {
+    double dacc[kNumSums];
+#pragma unroll
+    for (int k = 0; k < kNumSums; ++k) dacc[k] = k < NS ? dsum[k < NS ? k : 0][threadIdx.x] : 0.0;
+    block_write_sums<32 * NW>(dacc, a.partials, blockIdx.x);
+  }
 }
 
 // Runs per plane: enough warps for several full waves, while keeping the
@@ -702,7 +732,7 @@ static cudaError_t strip_launch_nw(const ProxArgs& a, int* nblocks_out, cudaStre
   constexpr int MINB = tvw_minb_nw<NTV, NORMS, NW>();
   // one ring a warp, and for the second part a 4-row ring of the stored duals
   constexpr size_t SMEM = Sh::SMEM / Sh::NW * NW + (PART == 2 ? (size_t)NW * 2 * 32 * 2 * sizeof(float4) : 0);
-  auto kern = k_prox_tv2d_strip<ST, NTV, NORMS, 2, NW, MINB, 4, 4, PART>;
+  auto kern = k_prox_tv2d_strip<ST, NTV, NORMS, 2, NW, MINB, PART>;
   cudaError_t e = allow_smem(kern, SMEM);
   if (e != cudaSuccess) return e;
   // resident blocks per SM, for the choice of runs per plane
