@@ -377,7 +377,10 @@ cudaError_t launch_holo_momentum(const float* dnew, float* dY0, float* dX, const
 // few SMs: the two inverse and two forward passes of the hologram, its pointwise
 // steps and their reductions were ten launches and a third of an iteration at
 // 128 x 128 x 32 (38 of 118 us; 54 of 276 at 384 x 384 x 40).  These two are
-// what is left of them in the loop.
+// what is left of them in the loop.  The sum of the z-chunks' spectra is bound by
+// latency: one part after another took 15 us at
+// 16 parts, and the steps of an iteration 25 us at 128 x 128 x 32 (22 us now)
+// and 29 us at 384 x 384 x 40 (26 us now).
 __global__ void __launch_bounds__(FLAT_THREADS) k_spec_residual(const float2* __restrict__ parts, int nparts,
                                                                 const float2* __restrict__ Bh,
                                                                 float2* __restrict__ Dn, int W, int H, SpecSums s) {
@@ -388,9 +391,21 @@ __global__ void __launch_bounds__(FLAT_THREADS) k_spec_residual(const float2* __
     const unsigned y = i / (unsigned)W, x = i - y * (unsigned)W;
     const unsigned p = (y ? H - y : 0) * (unsigned)W + (x ? W - x : 0);  // the element at -f
     float2 a = parts[i], b = parts[p];
-    for (int k = 1; k < nparts; ++k) {
-      a = cadd(a, parts[k * HW + i]);
-      b = cadd(b, parts[k * HW + p]);
+    // eight parts' loads in flight, added in order
+    for (int k0 = 1; k0 < nparts; k0 += 8) {
+      float2 va[8], vb[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (k0 + k < nparts) {
+          va[k] = parts[(k0 + k) * HW + i];
+          vb[k] = parts[(k0 + k) * HW + p];
+        }
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (k0 + k < nparts) {
+          a = cadd(a, va[k]);
+          b = cadd(b, vb[k]);
+        }
     }
     const float2 d = make_float2(0.5f * (a.x + b.x), 0.5f * (a.y - b.y));
     const bool pair = y > 0 && y < (unsigned)H / 2;  // else the partner's own thread writes it
