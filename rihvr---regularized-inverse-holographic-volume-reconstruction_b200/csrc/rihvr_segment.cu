@@ -52,6 +52,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <limits>
 #include <string>
 #include <type_traits>
 #include <vector>
@@ -88,14 +89,21 @@ __device__ __forceinline__ float q_from_value(float2 a) {
 // Voxel sources.  IntensitySrc: the intensities of a voxel file.  VolumeSrc:
 // the solver's volume x = P + beta (P - Pprev), formed on the fly as the
 // solver forms it, in the storage type of P.
+//
+// raw(i) is what the max and threshold passes look at: q itself, or the
+// intensity, of which q is a non-decreasing function (both its roundings are),
+// so that these passes need no square root a voxel.  -0 counts as 0; a
+// negative or NaN intensity, whose q is NaN, has the larger bit pattern.
 struct IntensitySrc {
   const float* I;
   __device__ __forceinline__ float q(size_t i) const { return q_from_intensity(__ldg(I + i)); }
+  __device__ __forceinline__ float raw(size_t i) const { return __ldg(I + i) + 0.f; }
 };
 // q values already formed (stored by the max pass)
 struct QSrc {
   const float* q_;
   __device__ __forceinline__ float q(size_t i) const { return __ldg(q_ + i); }
+  __device__ __forceinline__ float raw(size_t i) const { return __ldg(q_ + i); }
 };
 template <typename ST>
 struct VolumeSrc {
@@ -103,18 +111,19 @@ struct VolumeSrc {
   const ST* Pp;
   float beta;
   __device__ __forceinline__ float q(size_t i) const { return q_from_value(xval(P, Pp, beta, i)); }
+  __device__ __forceinline__ float raw(size_t i) const { return q(i); }
 };
 
-// largest q (non-negative floats order like their bit patterns); four
+// largest raw value (non-negative floats order like their bit patterns); four
 // independent loads a thread in flight
-// (qout, when given, receives every q for the threshold pass)
+// (qout, when given, receives every value for the threshold pass)
 template <typename SRC>
 __global__ void k_max_q(SRC src, unsigned long long n, unsigned* __restrict__ out_bits, float* __restrict__ qout) {
   unsigned m = 0;
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
   unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
   for (; i + 3 * stride < n; i += 4 * stride) {
-    const float a = src.q(i), b = src.q(i + stride), c = src.q(i + 2 * stride), e = src.q(i + 3 * stride);
+    const float a = src.raw(i), b = src.raw(i + stride), c = src.raw(i + 2 * stride), e = src.raw(i + 3 * stride);
     if (qout) {
       qout[i] = a;
       qout[i + stride] = b;
@@ -124,7 +133,7 @@ __global__ void k_max_q(SRC src, unsigned long long n, unsigned* __restrict__ ou
     m = max(m, max(max(__float_as_uint(a), __float_as_uint(b)), max(__float_as_uint(c), __float_as_uint(e))));
   }
   for (; i < n; i += stride) {
-    const float a = src.q(i);
+    const float a = src.raw(i);
     if (qout) qout[i] = a;
     m = max(m, __float_as_uint(a));
   }
@@ -133,11 +142,12 @@ __global__ void k_max_q(SRC src, unsigned long long n, unsigned* __restrict__ ou
 }
 
 // A warp makes eight words at a time (eight loads a lane in flight): lane b
-// holds voxel 32 w + b of its row; q > thr compared in FP64 as binarize_kernel
-// does (sparse_segmentation.cu:39-49).  Rows with a voxel on are flagged for
-// the morphology.
+// holds voxel 32 w + b of its row.  binarize_kernel compares q > thr in FP64
+// (sparse_segmentation.cu:39-49); `least` is the smallest raw value whose q
+// passes (NaN when none does), so one FP32 comparison gives the same bit.
+// Rows with a voxel on are flagged for the morphology.
 template <typename SRC>
-__global__ void k_binarize(SRC src, Dims d, double thr, unsigned* __restrict__ bits,
+__global__ void k_binarize(SRC src, Dims d, float least, unsigned* __restrict__ bits,
                            unsigned char* __restrict__ row_on) {
   constexpr int U = 8;
   const int lane = threadIdx.x & 31;
@@ -152,11 +162,11 @@ __global__ void k_binarize(SRC src, Dims d, double thr, unsigned* __restrict__ b
       const unsigned w = w0 + k;
       row[k] = w / WW;
       const int x = (int)(w - row[k] * WW) * 32 + lane;
-      q[k] = (w < nw && x < d.W) ? src.q((size_t)row[k] * d.W + x) : -1.f;
+      q[k] = (w < nw && x < d.W) ? src.raw((size_t)row[k] * d.W + x) : -1.f;
     }
 #pragma unroll
     for (int k = 0; k < U; ++k) {
-      const unsigned b = __ballot_sync(0xffffffffu, q[k] >= 0.f && (double)q[k] > thr);
+      const unsigned b = __ballot_sync(0xffffffffu, q[k] >= 0.f && q[k] >= least);
       const unsigned w = w0 + k;
       if (lane == 0 && w < nw) {
         bits[w] = b;
@@ -427,25 +437,35 @@ __global__ void k_finish(const int4* __restrict__ rec, const unsigned* __restric
   s.ymin = s.ymax = f.y;
   s.zmin = s.zmax = f.z;
   float vmax = __int_as_float(f.w);
-  for (unsigned j = j0; j < j1; ++j) {
-    const int4 e = rec[j];
-    const int x = e.x, y = e.y, z = e.z;
-    const float q = __int_as_float(e.w);
-    s.sx += x;
-    s.sy += y;
-    s.sz += z;
-    s.wsx = __fadd_rn(s.wsx, __fmul_rn(q, (float)x));
-    s.wsy = __fadd_rn(s.wsy, __fmul_rn(q, (float)y));
-    s.wsz = __fadd_rn(s.wsz, __fmul_rn(q, (float)z));
-    s.wsum = __fadd_rn(s.wsum, q);
-    s.vsum = __dadd_rn(s.vsum, (double)q);
-    vmax = q > vmax ? q : vmax;
-    s.xmin = min(s.xmin, x);
-    s.xmax = max(s.xmax, x);
-    s.ymin = min(s.ymin, y);
-    s.ymax = max(s.ymax, y);
-    s.zmin = min(s.zmin, z);
-    s.zmax = max(s.zmax, z);
+  // eight records ahead of the chain of additions, whose order is the reference's
+  constexpr unsigned AHEAD = 8;
+  int4 buf[AHEAD];
+  for (unsigned jb = j0; jb < j1; jb += AHEAD) {
+#pragma unroll
+    for (unsigned k = 0; k < AHEAD; ++k)
+      if (jb + k < j1) buf[k] = __ldg(rec + jb + k);
+#pragma unroll
+    for (unsigned k = 0; k < AHEAD; ++k) {
+      if (jb + k >= j1) break;
+      const int4 e = buf[k];
+      const int x = e.x, y = e.y, z = e.z;
+      const float q = __int_as_float(e.w);
+      s.sx += x;
+      s.sy += y;
+      s.sz += z;
+      s.wsx = __fadd_rn(s.wsx, __fmul_rn(q, (float)x));
+      s.wsy = __fadd_rn(s.wsy, __fmul_rn(q, (float)y));
+      s.wsz = __fadd_rn(s.wsz, __fmul_rn(q, (float)z));
+      s.wsum = __fadd_rn(s.wsum, q);
+      s.vsum = __dadd_rn(s.vsum, (double)q);
+      vmax = q > vmax ? q : vmax;
+      s.xmin = min(s.xmin, x);
+      s.xmax = max(s.xmax, x);
+      s.ymin = min(s.ymin, y);
+      s.ymax = max(s.ymax, y);
+      s.zmin = min(s.zmin, z);
+      s.zmax = max(s.zmax, z);
+    }
   }
   s.vmax = vmax;
   out[o] = s;
@@ -530,7 +550,7 @@ namespace rihvr {
 // sizes in three steps (the volume, the voxels that are on, the objects); the
 // buffers of a step are carved from one allocation.  One allocation a buffer,
 // some 25 of them with as many synchronising frees, had taken most of a
-// standalone call: 6.8 to 7.7 ms at 512 x 512 x 200 then, 3.0 to 3.5 ms now.
+// standalone call: 6.8 to 8.3 ms at 512 x 512 x 200 then, 2.1 ms now.
 struct SegWorkspace {
   static constexpr int kSteps = 3;
   unsigned char* p[kSteps] = {};
@@ -654,12 +674,16 @@ int segment_impl(SRC src, int W, int H, int Nz, const rihvr_segment_params* sp, 
   SegCarve c0;
   const size_t o_max = c0.add<unsigned>(1), o_err = c0.add<int>(1);
   const size_t o_bits0 = c0.add<unsigned>((size_t)d.nwords), o_bits1 = c0.add<unsigned>((size_t)d.nwords),
-               o_bits2 = c0.add<unsigned>((size_t)d.nwords), o_oncnt = c0.add<unsigned>((size_t)d.nwords),
+               o_bits2 = c0.add<unsigned>((size_t)d.nwords),
                o_onoff = c0.add<unsigned>((size_t)d.nwords + 1);
   const size_t o_row0 = c0.add<unsigned char>(nrows_vol), o_row1 = c0.add<unsigned char>(nrows_vol),
                o_row2 = c0.add<unsigned char>(nrows_vol);
   const size_t o_scan = c0.add<unsigned>(scan_scratch(d.nwords));
   const size_t o_q = kStoreQ ? c0.add<float>((size_t)nvox) : 0;
+  // room for the later steps when few voxels are on, as particles have it (one
+  // in 200; about 52 bytes each), so that a call allocates once
+  const size_t spare = 65536 + (size_t)nvox / 4;
+  const size_t o_spare = c0.add<unsigned char>(spare);
   SCK(ws.reserve(0, c0.bytes));
   unsigned char* const m0 = ws.p[0];
   unsigned* const maxbits = reinterpret_cast<unsigned*>(m0 + o_max);
@@ -667,7 +691,7 @@ int segment_impl(SRC src, int W, int H, int Nz, const rihvr_segment_params* sp, 
   unsigned* const bits0 = reinterpret_cast<unsigned*>(m0 + o_bits0);
   unsigned* const bits1 = reinterpret_cast<unsigned*>(m0 + o_bits1);
   unsigned* const bits2 = reinterpret_cast<unsigned*>(m0 + o_bits2);
-  unsigned* const oncnt = reinterpret_cast<unsigned*>(m0 + o_oncnt);
+  unsigned* const oncnt = bits1;  // the dilated volume is done with when the counts are made
   unsigned* const onoff = reinterpret_cast<unsigned*>(m0 + o_onoff);
   unsigned char *const row0 = m0 + o_row0, *const row1 = m0 + o_row1, *const row2 = m0 + o_row2;
   unsigned* const scan0 = reinterpret_cast<unsigned*>(m0 + o_scan);
@@ -684,16 +708,41 @@ int segment_impl(SRC src, int W, int H, int Nz, const rihvr_segment_params* sp, 
   k_max_q<<<grid_for((long long)nvox, 256), 256, 0, st>>>(src, nvox, maxbits, qbuf);
   SCK(cudaGetLastError());
   ++launches;
+  // a value's q on the host (the same IEEE operations)
+  const auto q_of = [](float v) {
+    if (kStoreQ) return v;
+    const float r = std::sqrt(v);
+    return r * r;
+  };
   unsigned mb = 0;
   SCK(cudaMemcpyAsync(&mb, maxbits, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
   SCK(cudaStreamSynchronize(st));
-  float maxq;
-  std::memcpy(&maxq, &mb, sizeof(float));
+  float maxq = std::numeric_limits<float>::quiet_NaN();  // a negative or NaN value: no q is the largest
+  if (mb <= 0x7f800000u) {
+    std::memcpy(&maxq, &mb, sizeof(float));
+    maxq = q_of(maxq);
+  }
   const double thr = sp->min_intensity * (double)maxq / 256.0;
+  // smallest raw value whose q passes the threshold, by bisection of the bit patterns 0 .. +inf
+  float least = std::numeric_limits<float>::quiet_NaN();
+  const auto passes = [&](unsigned bits) {
+    float v;
+    std::memcpy(&v, &bits, sizeof(float));
+    return (double)q_of(v) > thr;
+  };
+  if (passes(0x7f800000u)) {
+    unsigned lo = 0, hi = 0x7f800000u;  // hi passes
+    while (lo < hi) {
+      const unsigned mid = lo + (hi - lo) / 2;
+      if (passes(mid)) hi = mid;
+      else lo = mid + 1;
+    }
+    std::memcpy(&least, &hi, sizeof(float));
+  }
   if (kStoreQ)
-    k_binarize<<<grid_for(d.nwords * 4, 256), 256, 0, st>>>(QSrc{qbuf}, d, thr, bits0, row0);
+    k_binarize<<<grid_for(d.nwords * 4, 256), 256, 0, st>>>(QSrc{qbuf}, d, least, bits0, row0);
   else
-    k_binarize<<<grid_for(d.nwords * 4, 256), 256, 0, st>>>(src, d, thr, bits0, row0);
+    k_binarize<<<grid_for(d.nwords * 4, 256), 256, 0, st>>>(src, d, least, bits0, row0);
   SCK(cudaGetLastError());
   ++launches;
 
@@ -736,8 +785,9 @@ int segment_impl(SRC src, int W, int H, int Nz, const rihvr_segment_params* sp, 
                  o_val = c1.add<unsigned>(non), o_keys = c1.add<unsigned>(non), o_vals = c1.add<unsigned>(non),
                  o_rec = c1.add<int4>(non), o_scan1 = c1.add<unsigned>(scan_scratch(non)),
                  o_tmp = c1.add<unsigned char>(tmp_bytes);
-    SCK(ws.reserve(1, c1.bytes));
-    unsigned char* const m1 = ws.p[1];
+    const bool spare1 = c1.bytes <= spare;
+    if (!spare1) SCK(ws.reserve(1, c1.bytes));
+    unsigned char* const m1 = spare1 ? m0 + o_spare : ws.p[1];
     unsigned* const idx = reinterpret_cast<unsigned*>(m1 + o_idx);
     unsigned* const lab = reinterpret_cast<unsigned*>(m1 + o_lab);
     unsigned* const is_root = reinterpret_cast<unsigned*>(m1 + o_root);
@@ -771,8 +821,9 @@ int segment_impl(SRC src, int W, int H, int Nz, const rihvr_segment_params* sp, 
     SegCarve c2;
     const size_t o_cnt = c2.add<unsigned>(nobj), o_off = c2.add<unsigned>((size_t)nobj + 1),
                  o_sums = c2.add<ObjSums>(nobj), o_scan2 = c2.add<unsigned>(scan_scratch(nobj));
-    SCK(ws.reserve(2, c2.bytes));
-    unsigned char* const m2 = ws.p[2];
+    const bool spare2 = (spare1 ? c1.bytes : 0) + c2.bytes <= spare;
+    if (!spare2) SCK(ws.reserve(2, c2.bytes));
+    unsigned char* const m2 = spare2 ? m0 + o_spare + (spare1 ? c1.bytes : 0) : ws.p[2];
     unsigned* const cnt = reinterpret_cast<unsigned*>(m2 + o_cnt);
     unsigned* const off = reinterpret_cast<unsigned*>(m2 + o_off);
     ObjSums* const osum = reinterpret_cast<ObjSums*>(m2 + o_sums);
