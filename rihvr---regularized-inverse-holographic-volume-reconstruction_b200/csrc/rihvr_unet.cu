@@ -260,51 +260,83 @@ cudaError_t conv3(const float* X, int Cin, const __nv_bfloat16* Wt, int Cout, in
   }
 }
 
-// db[co] += sum_v dY[v][co]
-__global__ void k_bias_grad(const float* __restrict__ dY, int C, long long n, float* __restrict__ db) {
-  __shared__ float part[64];
-  if (threadIdx.x < 64) part[threadIdx.x] = 0.f;
-  __syncthreads();
-  const int c = threadIdx.x % C;
-  const int lanes = blockDim.x / C;
-  float s = 0.f;
-  for (long long vv = (long long)blockIdx.x * lanes + threadIdx.x / C; vv < n; vv += (long long)gridDim.x * lanes)
-    if (threadIdx.x < lanes * C) s += dY[vv * C + c];
-  if (threadIdx.x < lanes * C) atomicAdd(&part[c], s);
-  __syncthreads();
-  if (threadIdx.x < C) atomicAdd(&db[threadIdx.x], part[threadIdx.x]);
+// The elementwise passes below walk rows of voxels (a block a (z, y) row, 4 or
+// 8 channels a thread), so that only 32-bit divisions by the channel count are
+// left inside; with a 64-bit division chain for every element they had taken
+// more time than their bytes: 137 us instead of 30 us for the up-and-concatenate
+// of a 32 x 128 x 128 volume.
+
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ float4 add4(float4 a, float4 b) {
+  return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
 }
 
-// dY *= (Y > 0): through the ReLU whose output is Y
-__global__ void k_relu_back(float* __restrict__ dY, const float* __restrict__ Y, long long n) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    if (!(Y[i] > 0.f)) dY[i] = 0.f;
+// dY *= (Y > 0), through the ReLU whose output is Y, and db[co] += sum_v dY[v][co]
+// of what is left.  C is 16, 32 or 64: a thread keeps its 4 channels.
+__global__ void __launch_bounds__(256) k_relu_bias_back(float* __restrict__ dY, const float* __restrict__ Y, int C,
+                                                        long long n, float* __restrict__ db) {
+  __shared__ float4 part[256];
+  const int G = C / 4;
+  const long long total = n * G;  // groups of 4 channels; the stride is a multiple of G
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (long long e = (long long)blockIdx.x * 256 + threadIdx.x; e < total; e += (long long)gridDim.x * 256) {
+    const float4 y = ld4(Y + 4 * e);
+    float4 d = ld4(dY + 4 * e);
+    d.x = y.x > 0.f ? d.x : 0.f;
+    d.y = y.y > 0.f ? d.y : 0.f;
+    d.z = y.z > 0.f ? d.z : 0.f;
+    d.w = y.w > 0.f ? d.w : 0.f;
+    st4(dY + 4 * e, d);
+    s = add4(s, d);
+  }
+  part[threadIdx.x] = s;
+  __syncthreads();
+  for (int h = 128; h >= G; h >>= 1) {  // G is a power of two: partners hold the same channels
+    if (threadIdx.x < h) part[threadIdx.x] = add4(part[threadIdx.x], part[threadIdx.x + h]);
+    __syncthreads();
+  }
+  if ((int)threadIdx.x < G) {
+    const float4 t = part[threadIdx.x];
+    float* d = db + 4 * threadIdx.x;
+    atomicAdd(d, t.x);
+    atomicAdd(d + 1, t.y);
+    atomicAdd(d + 2, t.z);
+    atomicAdd(d + 3, t.w);
+  }
 }
 
 // 2x2x2 average pool (fine volume f, coarse c) and its gradient
 __global__ void k_pool(const float* __restrict__ X, float* __restrict__ Y, Vol c, int C) {
-  const long long n = c.n() * C;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    const int ch = (int)(e % C);
-    const long long vv = e / C;
-    const int x = (int)(vv % c.W), y = (int)((vv / c.W) % c.H), z = (int)(vv / ((long long)c.W * c.H));
-    const int W2 = 2 * c.W, H2 = 2 * c.H;
-    float s = 0.f;
+  const int G = C / 4, W2 = 2 * c.W, H2 = 2 * c.H;
+  for (int row = blockIdx.x; row < c.D * c.H; row += gridDim.x) {
+    const int z = row / c.H, y = row - z * c.H;
+    for (int e = threadIdx.x; e < c.W * G; e += blockDim.x) {
+      const int x = e / G, g = e - x * G;
+      float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
-      s += X[((((long long)(2 * z + (q >> 2)) * H2 + 2 * y + ((q >> 1) & 1)) * W2) + 2 * x + (q & 1)) * C + ch];
-    Y[e] = s * 0.125f;
+      for (int q = 0; q < 8; ++q)
+        s = add4(s, ld4(X + ((((long long)(2 * z + (q >> 2)) * H2 + 2 * y + ((q >> 1) & 1)) * W2) + 2 * x + (q & 1)) * C +
+                        4 * g));
+      st4(Y + ((long long)row * c.W + x) * C + 4 * g,
+          make_float4(s.x * 0.125f, s.y * 0.125f, s.z * 0.125f, s.w * 0.125f));
+    }
   }
 }
 // dX = (gradient through the pool) + S, S the skip gradient of the same tensor
 __global__ void k_pool_back(const float* __restrict__ dY, const float* __restrict__ S, float* __restrict__ dX,
                             Vol f, int C) {
-  const long long n = f.n() * C;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    const int ch = (int)(e % C);
-    const long long vv = e / C;
-    const int x = (int)(vv % f.W), y = (int)((vv / f.W) % f.H), z = (int)(vv / ((long long)f.W * f.H));
-    dX[e] = 0.125f * dY[((((long long)(z >> 1) * (f.H >> 1)) + (y >> 1)) * (f.W >> 1) + (x >> 1)) * C + ch] + S[e];
+  const int G = C / 4;
+  for (int row = blockIdx.x; row < f.D * f.H; row += gridDim.x) {
+    const int z = row / f.H, y = row - z * f.H;
+    const float* src = dY + (((long long)(z >> 1) * (f.H >> 1)) + (y >> 1)) * (f.W >> 1) * C;
+    const long long base = (long long)row * f.W * C;
+    for (int e = threadIdx.x; e < f.W * G; e += blockDim.x) {
+      const int x = e / G, g = e - x * G;
+      const float4 d = ld4(src + (long long)(x >> 1) * C + 4 * g), s = ld4(S + base + 4 * e);
+      st4(dX + base + 4 * e,
+          make_float4(0.125f * d.x + s.x, 0.125f * d.y + s.y, 0.125f * d.z + s.z, 0.125f * d.w + s.w));
+    }
   }
 }
 
@@ -312,16 +344,15 @@ __global__ void k_pool_back(const float* __restrict__ dY, const float* __restric
 // channel tensor whose channels [Cu, Cu + Cs) are the skip tensor S
 __global__ void k_up_concat(const float* __restrict__ U, int Cu, const float* __restrict__ S, int Cs,
                             float* __restrict__ Y, Vol f) {
-  const int C = Cu + Cs;
-  const long long n = f.n() * C;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    const int ch = (int)(e % C);
-    const long long vv = e / C;
-    if (ch >= Cu) {
-      Y[e] = S[vv * Cs + ch - Cu];
-    } else {
-      const int x = (int)(vv % f.W), y = (int)((vv / f.W) % f.H), z = (int)(vv / ((long long)f.W * f.H));
-      Y[e] = U[((((long long)(z >> 1) * (f.H >> 1)) + (y >> 1)) * (f.W >> 1) + (x >> 1)) * Cu + ch];
+  const int C = Cu + Cs, G = C / 4;
+  for (int row = blockIdx.x; row < f.D * f.H; row += gridDim.x) {
+    const int z = row / f.H, y = row - z * f.H;
+    const float* src = U + (((long long)(z >> 1) * (f.H >> 1)) + (y >> 1)) * (f.W >> 1) * Cu;
+    for (int e = threadIdx.x; e < f.W * G; e += blockDim.x) {
+      const int x = e / G, ch = 4 * (e - x * G);
+      const float4 v = ch >= Cu ? ld4(S + ((long long)row * f.W + x) * Cs + ch - Cu)
+                                : ld4(src + (long long)(x >> 1) * Cu + ch);
+      st4(Y + (long long)row * f.W * C + 4 * e, v);
     }
   }
 }
@@ -329,24 +360,26 @@ __global__ void k_up_concat(const float* __restrict__ U, int Cu, const float* __
 // dS = channels [Cu, Cu + Cs)
 __global__ void k_up_concat_back(const float* __restrict__ dY, int Cu, int Cs, float* __restrict__ dU,
                                  float* __restrict__ dS, Vol c) {
-  const int C = Cu + Cs;
+  const int C = Cu + Cs, Gu = Cu / 4, Gs = Cs / 4;
   const int W2 = 2 * c.W, H2 = 2 * c.H;
-  const long long nu = c.n() * Cu;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < nu; e += (long long)gridDim.x * blockDim.x) {
-    const int ch = (int)(e % Cu);
-    const long long vv = e / Cu;
-    const int x = (int)(vv % c.W), y = (int)((vv / c.W) % c.H), z = (int)(vv / ((long long)c.W * c.H));
-    float s = 0.f;
+  for (int row = blockIdx.x; row < c.D * c.H; row += gridDim.x) {
+    const int z = row / c.H, y = row - z * c.H;
+    for (int e = threadIdx.x; e < c.W * Gu; e += blockDim.x) {
+      const int x = e / Gu, g = e - x * Gu;
+      float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
-      s += dY[((((long long)(2 * z + (q >> 2)) * H2 + 2 * y + ((q >> 1) & 1)) * W2) + 2 * x + (q & 1)) * C + ch];
-    dU[e] = s;
-  }
-  const long long ns = c.n() * 8 * Cs;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < ns; e += (long long)gridDim.x * blockDim.x) {
-    const int ch = (int)(e % Cs);
-    const long long vv = e / Cs;
-    dS[e] = dY[vv * C + Cu + ch];
+      for (int q = 0; q < 8; ++q)
+        s = add4(s, ld4(dY + ((((long long)(2 * z + (q >> 2)) * H2 + 2 * y + ((q >> 1) & 1)) * W2) + 2 * x + (q & 1)) * C +
+                        4 * g));
+      st4(dU + ((long long)row * c.W + x) * Cu + 4 * g, s);
+    }
+    for (int q = 0; q < 4; ++q) {  // the four fine rows of the coarse one
+      const long long fr = (long long)(2 * z + (q >> 1)) * H2 + 2 * y + (q & 1);
+      for (int e = threadIdx.x; e < W2 * Gs; e += blockDim.x) {
+        const int x = e / Gs, g = e - x * Gs;
+        st4(dS + (fr * W2 + x) * Cs + 4 * g, ld4(dY + (fr * W2 + x) * C + Cu + 4 * g));
+      }
+    }
   }
 }
 
@@ -362,7 +395,8 @@ __global__ void k_input(const float2* __restrict__ xbp, long long n, const float
   }
 }
 
-// sum |xbp|^2 (FP64 partials into out[0]) and sum |x*|^2 (out[1])
+// sum |xbp|^2 (FP64 partials into out[0]) and sum |x*|^2 (out[1]); 256 threads,
+// one atomic a block
 __global__ void k_sumsq(const float2* __restrict__ a, const float2* __restrict__ b, long long n,
                         double* __restrict__ out) {
   double sa = 0, sb = 0;
@@ -374,13 +408,20 @@ __global__ void k_sumsq(const float2* __restrict__ a, const float2* __restrict__
       sb += (double)q.x * q.x + (double)q.y * q.y;
     }
   }
+  __shared__ double red[2][8];
   for (int o = 16; o; o >>= 1) {
     sa += __shfl_xor_sync(0xffffffffu, sa, o);
     sb += __shfl_xor_sync(0xffffffffu, sb, o);
   }
   if ((threadIdx.x & 31) == 0) {
-    atomicAdd(out, sa);
-    if (b) atomicAdd(out + 1, sb);
+    red[0][threadIdx.x >> 5] = sa;
+    red[1][threadIdx.x >> 5] = sb;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2 && (threadIdx.x == 0 || b)) {
+    double s = 0;
+    for (unsigned w = 0; w < blockDim.x / 32; ++w) s += red[threadIdx.x][w];
+    atomicAdd(out + threadIdx.x, s);
   }
 }
 __global__ void k_rms(const double* __restrict__ s, long long n, float* __restrict__ rms) {
@@ -403,11 +444,11 @@ __global__ void k_head(const float* __restrict__ Hh, const float* __restrict__ w
 }
 
 // loss = sum |x0 - x*|^2 / S* and the gradients: dz[v] (through the sigmoid),
-// head weights/bias and alpha (FP32 atomics into dw[0..17]), loss (FP64)
+// head weights/bias and alpha (FP32 sums a warp, parts[18][warps]), loss (FP64)
 __global__ void k_head_back(const float* __restrict__ Hh, const float* __restrict__ w,
                             const float2* __restrict__ xbp, const float2* __restrict__ xs,
                             const float* __restrict__ gbuf, long long n, const double* __restrict__ sums,
-                            float* __restrict__ dH, float* __restrict__ dw, double* __restrict__ loss) {
+                            float* __restrict__ dH, float* __restrict__ parts, double* __restrict__ loss) {
   const float alpha = w[17];
   const double Sstar = fmax(sums[1], 1e-300);
   const float inv = (float)(1.0 / Sstar);
@@ -431,16 +472,62 @@ __global__ void k_head_back(const float* __restrict__ Hh, const float* __restric
       dH[i * 16 + c] = dz * w[c];
     }
   }
+  __shared__ double redl[8];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int nw = gridDim.x * (blockDim.x / 32), wi = blockIdx.x * (blockDim.x / 32) + wid;
   for (int o = 16; o; o >>= 1) {
     l += __shfl_xor_sync(0xffffffffu, l, o);
 #pragma unroll
     for (int c = 0; c < 18; ++c) dwl[c] += __shfl_xor_sync(0xffffffffu, dwl[c], o);
   }
-  if ((threadIdx.x & 31) == 0) {
-    atomicAdd(loss, l / Sstar);
+  if (lane == 0) {
+    redl[wid] = l;
 #pragma unroll
-    for (int c = 0; c < 18; ++c) atomicAdd(&dw[c], dwl[c]);
+    for (int c = 0; c < 18; ++c) parts[(size_t)c * nw + wi] = dwl[c];
   }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0;
+    for (unsigned k = 0; k < blockDim.x / 32; ++k) s += redl[k];
+    atomicAdd(loss, s / Sstar);
+  }
+}
+
+// dw[c] += the warps' sums, one block a sum, added one after another in warp
+// order by one thread.  An empty volume's voxels all add the same value, and a
+// chain rounds every such addition alike (2e-5 of the largest sum at
+// 32 x 128 x 128, against a tree); this is the chain that an atomic add a warp makes, which had taken
+// nine tenths of the kernel above (315 us; 54 us without it), in
+// 47 us.
+__global__ void k_head_sums(const float* __restrict__ parts, int nw, float* __restrict__ dw) {
+  constexpr int CH = 2048;  // values staged at a time; zeros past the end do not change a sum
+  __shared__ float4 st[CH / 4];
+  const float* p = parts + (size_t)blockIdx.x * nw;
+  float s = 0.f;
+  for (int b = 0; b < nw; b += CH) {
+    __syncthreads();
+    for (int k = threadIdx.x; k < CH; k += blockDim.x)
+      reinterpret_cast<float*>(st)[k] = b + k < nw ? p[b + k] : 0.f;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      float4 q[4], n[4];  // the next 16 values are read while these are added
+#pragma unroll
+      for (int k = 0; k < 4; ++k) q[k] = st[k];
+      for (int k0 = 4; k0 <= CH / 4; k0 += 4) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) n[k] = st[k0 < CH / 4 ? k0 + k : k];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          s += q[k].x;
+          s += q[k].y;
+          s += q[k].z;
+          s += q[k].w;
+          q[k] = n[k];
+        }
+      }
+    }
+  }
+  if (threadIdx.x == 0) dw[blockIdx.x] += s;
 }
 
 // Adam (FP32 masters) and the BF16 copies the convolutions read; the
@@ -522,24 +609,20 @@ __global__ void k_pool_bf16(const __nv_bfloat16* __restrict__ X, __nv_bfloat16* 
   }
 }
 
-// nearest x2 upsampling of U (Cu channels) and concatenation with S (Cs), 8
-// channels a thread
-__global__ void k_up_concat_bf16(const __nv_bfloat16* __restrict__ U, int Cu, const __nv_bfloat16* __restrict__ S,
-                                 int Cs, __nv_bfloat16* __restrict__ Y, Vol f) {
-  const int C = Cu + Cs, G = C / 8;
-  const long long n = f.n() * G;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    const int g = (int)(e % G);
-    const long long vv = e / G;
-    uint4 v;
-    if (g * 8 >= Cu) {
-      v = *reinterpret_cast<const uint4*>(S + vv * Cs + g * 8 - Cu);
-    } else {
-      const int x = (int)(vv % f.W), y = (int)((vv / f.W) % f.H), z = (int)(vv / ((long long)f.W * f.H));
-      const long long src = (((long long)(z >> 1) * (f.H >> 1)) + (y >> 1)) * (f.W >> 1) + (x >> 1);
-      v = *reinterpret_cast<const uint4*>(U + src * Cu + g * 8);
+// nearest x2 upsampling of U (C channels, 8 a thread); the convolution that
+// follows reads the skip tensor where it lies
+__global__ void k_up_bf16(const __nv_bfloat16* __restrict__ U, int C, __nv_bfloat16* __restrict__ Y, Vol f) {
+  const int G = C / 8;
+  for (int row = blockIdx.x; row < f.D * f.H; row += gridDim.x) {
+    const int z = row / f.H, y = row - z * f.H;
+    const __nv_bfloat16* src = U + (((long long)(z >> 1) * (f.H >> 1)) + (y >> 1)) * (f.W >> 1) * C;
+    __nv_bfloat16* dst = Y + (long long)row * f.W * C;
+    for (int e = threadIdx.x; e < (f.W >> 1) * G; e += blockDim.x) {  // a coarse voxel's group, stored twice
+      const int x = e / G, g = e - x * G;
+      const uint4 v = *reinterpret_cast<const uint4*>(src + (long long)x * C + g * 8);
+      *reinterpret_cast<uint4*>(dst + (long long)(2 * x) * C + g * 8) = v;
+      *reinterpret_cast<uint4*>(dst + (long long)(2 * x + 1) * C + g * 8) = v;
     }
-    *reinterpret_cast<uint4*>(Y + vv * C + g * 8) = v;
   }
 }
 
@@ -568,6 +651,9 @@ int blocks_for(long long n, int threads = 256) {
   const long long b = (n + threads - 1) / threads;
   return (int)std::max<long long>(1, std::min<long long>(b, 148LL * 32));
 }
+
+// a block a (z, y) row of a volume, for the passes that walk rows
+int rows_of(const Vol& v) { return (int)std::min<long long>((long long)v.D * v.H, 1 << 30); }
 
 // one 3x3x3 convolution layer
 struct Conv {
@@ -617,8 +703,11 @@ struct rihvr_unet {
   __nv_bfloat16 *b_p1 = nullptr, *b_a2 = nullptr, *b_a3 = nullptr, *b_c2 = nullptr, *b_a7 = nullptr;  // level 1
   __nv_bfloat16 *b_p2 = nullptr, *b_a4 = nullptr, *b_a5 = nullptr;  // level 2
   TcMap maps[kNumConv];
+  TcMap skip_maps[kNumConv] = {};  // the skip tensor of a decoder's first layer
+  int cin_a[kNumConv] = {};        // input channels of `maps`; the others are the skip tensor's
   TcMap zmaps[kNumConv];  // the z-walking form's maps, where a layer takes it
   bool zwalk[kNumConv] = {};
+  float* head_parts = nullptr;  // warps' sums of the head's gradient
   double* sums = nullptr;   // [0] sum |xbp|^2, [1] sum |x*|^2, [2] loss
   int* tc_err = nullptr;    // set by a tcgen05 convolution whose bounded wait ran out
   float* rms = nullptr;
@@ -657,10 +746,10 @@ int conv_back(rihvr_unet* u, int li, const float* X, float* dY, float* dX) {
   const Conv& L = u->layers[li];
   const Vol v = u->lv[L.level];
   const long long n = v.n();
-  k_relu_back<<<blocks_for(n * L.cout), 256, 0, u->st>>>(dY, u->act[li], n * L.cout);
+  k_relu_bias_back<<<(unsigned)std::min<long long>(148 * 4, (n * (L.cout / 4) + 255) / 256), 256, 0, u->st>>>(
+      dY, u->act[li], L.cout, n, u->gw + L.b_off);
   UCK(conv3_wgrad(X, L.cin, dY, L.cout, u->gw + L.w_off, v.D, v.H, v.W, u->st));
-  k_bias_grad<<<(unsigned)std::min<long long>(1024, (n + 7) / 8), 256, 0, u->st>>>(dY, L.cout, n, u->gw + L.b_off);
-  u->launches += 3;
+  u->launches += 2;
   // the data gradient: output channels of the transposed weights in windows of 64
   for (int co0 = 0; dX && co0 < L.cin; co0 += 64) {
     UCK(conv3(dY, L.cout, u->wt + u->wb_off[li], L.cin, co0, std::min(64, L.cin - co0), nullptr, dX, v, 0, 1,
@@ -688,19 +777,19 @@ int refresh_bf16(rihvr_unet* u) {
 int forward(rihvr_unet* u, const float2* xbp, const float2* xs, float2* x0, float scale = 1.f) {
   const long long n0 = u->lv[0].n();
   UCK(cudaMemsetAsync(u->sums, 0, 3 * sizeof(double), u->st));
-  k_sumsq<<<blocks_for(n0), 256, 0, u->st>>>(xbp, xs, n0, u->sums);
+  k_sumsq<<<(int)std::min<long long>(148 * 8, blocks_for(n0)), 256, 0, u->st>>>(xbp, xs, n0, u->sums);
   k_rms<<<1, 1, 0, u->st>>>(u->sums, n0, u->rms);
   k_input<<<blocks_for(n0), 256, 0, u->st>>>(xbp, n0, u->rms, u->in0);
   u->launches += 3;
   int rc;
   if ((rc = conv_fwd(u, 0, u->in0, u->act[0])) || (rc = conv_fwd(u, 1, u->act[0], u->act[1]))) return rc;
-  k_pool<<<blocks_for(u->lv[1].n() * 16), 256, 0, u->st>>>(u->act[1], u->p1, u->lv[1], 16);
+  k_pool<<<rows_of(u->lv[1]), 256, 0, u->st>>>(u->act[1], u->p1, u->lv[1], 16);
   if ((rc = conv_fwd(u, 2, u->p1, u->act[2])) || (rc = conv_fwd(u, 3, u->act[2], u->act[3]))) return rc;
-  k_pool<<<blocks_for(u->lv[2].n() * 32), 256, 0, u->st>>>(u->act[3], u->p2, u->lv[2], 32);
+  k_pool<<<rows_of(u->lv[2]), 256, 0, u->st>>>(u->act[3], u->p2, u->lv[2], 32);
   if ((rc = conv_fwd(u, 4, u->p2, u->act[4])) || (rc = conv_fwd(u, 5, u->act[4], u->act[5]))) return rc;
-  k_up_concat<<<blocks_for(u->lv[1].n() * 96), 256, 0, u->st>>>(u->act[5], 64, u->act[3], 32, u->c2, u->lv[1]);
+  k_up_concat<<<rows_of(u->lv[1]), 256, 0, u->st>>>(u->act[5], 64, u->act[3], 32, u->c2, u->lv[1]);
   if ((rc = conv_fwd(u, 6, u->c2, u->act[6])) || (rc = conv_fwd(u, 7, u->act[6], u->act[7]))) return rc;
-  k_up_concat<<<blocks_for(n0 * 48), 256, 0, u->st>>>(u->act[7], 32, u->act[1], 16, u->c1, u->lv[0]);
+  k_up_concat<<<rows_of(u->lv[0]), 256, 0, u->st>>>(u->act[7], 32, u->act[1], 16, u->c1, u->lv[0]);
   if ((rc = conv_fwd(u, 8, u->c1, u->act[8])) || (rc = conv_fwd(u, 9, u->act[8], u->act[9]))) return rc;
   k_head<<<blocks_for(n0), 256, 0, u->st>>>(u->act[9], u->w + u->head_off, xbp, n0, scale, u->gbuf, x0);
   u->launches += 5;
@@ -712,22 +801,25 @@ int forward(rihvr_unet* u, const float2* xbp, const float2* xs, float2* x0, floa
 int backward(rihvr_unet* u, const float2* xbp, const float2* xs) {
   const long long n0 = u->lv[0].n(), n1 = u->lv[1].n();
   UCK(cudaMemsetAsync(u->gw, 0, sizeof(float) * u->nparam, u->st));
-  k_head_back<<<blocks_for(n0), 256, 0, u->st>>>(u->act[9], u->w + u->head_off, xbp, xs, u->gbuf, n0, u->sums,
-                                                u->A0a, u->gw + u->head_off, u->sums + 2);
+  const int hb = blocks_for(n0);
+  k_head_back<<<hb, 256, 0, u->st>>>(u->act[9], u->w + u->head_off, xbp, xs, u->gbuf, n0, u->sums, u->A0a,
+                                     u->head_parts, u->sums + 2);
+  k_head_sums<<<18, 256, 0, u->st>>>(u->head_parts, hb * 8, u->gw + u->head_off);
+  ++u->launches;
   ++u->launches;
   int rc;
   if ((rc = conv_back(u, 9, u->act[8], u->A0a, u->A0b))) return rc;  // dec1b
   if ((rc = conv_back(u, 8, u->c1, u->A0b, u->C0))) return rc;        // dec1a: 48 ch
-  k_up_concat_back<<<blocks_for(n0 * 16), 256, 0, u->st>>>(u->C0, 32, 16, u->B1a, u->S0, u->lv[1]);
+  k_up_concat_back<<<rows_of(u->lv[1]), 256, 0, u->st>>>(u->C0, 32, 16, u->B1a, u->S0, u->lv[1]);
   if ((rc = conv_back(u, 7, u->act[6], u->B1a, u->B1b))) return rc;  // dec2b
   if ((rc = conv_back(u, 6, u->c2, u->B1b, u->C1))) return rc;        // dec2a: 96 ch
-  k_up_concat_back<<<blocks_for(n1 * 32), 256, 0, u->st>>>(u->C1, 64, 32, u->D2a, u->S1, u->lv[2]);
+  k_up_concat_back<<<rows_of(u->lv[2]), 256, 0, u->st>>>(u->C1, 64, 32, u->D2a, u->S1, u->lv[2]);
   if ((rc = conv_back(u, 5, u->act[4], u->D2a, u->D2b))) return rc;  // bottom b
   if ((rc = conv_back(u, 4, u->p2, u->D2b, u->P2))) return rc;        // bottom a
-  k_pool_back<<<blocks_for(n1 * 32), 256, 0, u->st>>>(u->P2, u->S1, u->B1a, u->lv[1], 32);
+  k_pool_back<<<rows_of(u->lv[1]), 256, 0, u->st>>>(u->P2, u->S1, u->B1a, u->lv[1], 32);
   if ((rc = conv_back(u, 3, u->act[2], u->B1a, u->B1b))) return rc;  // enc2b
   if ((rc = conv_back(u, 2, u->p1, u->B1b, u->P1))) return rc;        // enc2a
-  k_pool_back<<<blocks_for(n0 * 16), 256, 0, u->st>>>(u->P1, u->S0, u->A0a, u->lv[0], 16);
+  k_pool_back<<<rows_of(u->lv[0]), 256, 0, u->st>>>(u->P1, u->S0, u->A0a, u->lv[0], 16);
   if ((rc = conv_back(u, 1, u->act[0], u->A0a, u->A0b))) return rc;  // enc1b
   if ((rc = conv_back(u, 0, u->in0, u->A0b, nullptr))) return rc;     // enc1a
   u->launches += 4;
@@ -759,11 +851,11 @@ int bf16_prepare(rihvr_unet* u) {
   A(&u->b_in0, n0 * 16);
   A(&u->b_a0, n0 * 16);
   A(&u->b_a1, n0 * 16);
-  A(&u->b_c1, n0 * 48);
+  A(&u->b_c1, n0 * 32);
   A(&u->b_p1, n1 * 16);
   A(&u->b_a2, n1 * 32);
   A(&u->b_a3, n1 * 32);
-  A(&u->b_c2, n1 * 96);
+  A(&u->b_c2, n1 * 64);
   A(&u->b_a7, n1 * 32);
   A(&u->b_p2, n2 * 32);
   A(&u->b_a4, n2 * 64);
@@ -776,7 +868,11 @@ int bf16_prepare(rihvr_unet* u) {
   for (int i = 0; i < kNumConv; ++i) {
     const Conv& L = u->layers[i];
     const Vol v = u->lv[L.level];
-    if (!tc_map_encode(&u->maps[i], in[i], L.cin, v.D, v.H, v.W)) {
+    // the decoders' first layers read an upsampled tensor and, after it, a skip tensor
+    const int cskip = i == 6 ? 32 : i == 8 ? 16 : 0;
+    u->cin_a[i] = L.cin - cskip;
+    if (!tc_map_encode(&u->maps[i], in[i], u->cin_a[i], v.D, v.H, v.W) ||
+        (cskip && !tc_map_encode(&u->skip_maps[i], i == 6 ? u->b_a3 : u->b_a1, cskip, v.D, v.H, v.W))) {
       u->bf_failed = true;
       return RIHVR_OK;
     }
@@ -794,7 +890,7 @@ int conv_bf16(rihvr_unet* u, int li, __nv_bfloat16* Y, const TcHead* head = null
     UCK(conv3_tcz(u->zmaps[li], L.cin, u->wtc + u->wtc_off[li], u->w + L.b_off, L.cout, Y, v.D, v.H, v.W, head,
                   u->tc_err, u->st));
   else
-    UCK(conv3_tc_bf16(u->maps[li], L.cin, u->wtc + u->wtc_off[li], u->w + L.b_off, L.cout, Y, v.D, v.H, v.W, head,
+    UCK(conv3_tc_bf16(u->maps[li], u->skip_maps[li], u->cin_a[li], L.cin, u->wtc + u->wtc_off[li], u->w + L.b_off, L.cout, Y, v.D, v.H, v.W, head,
                       u->tc_err, u->st));
   ++u->launches;
   return RIHVR_OK;
@@ -809,7 +905,7 @@ int forward_bf16(rihvr_unet* u, const float2* xbp, float2* x0, float scale) {
   if (rc != RIHVR_OK) return rc;
   const long long n0 = u->lv[0].n(), n1 = u->lv[1].n(), n2 = u->lv[2].n();
   UCK(cudaMemsetAsync(u->sums, 0, 3 * sizeof(double), u->st));
-  k_sumsq<<<blocks_for(n0), 256, 0, u->st>>>(xbp, nullptr, n0, u->sums);
+  k_sumsq<<<(int)std::min<long long>(148 * 8, blocks_for(n0)), 256, 0, u->st>>>(xbp, nullptr, n0, u->sums);
   k_rms<<<1, 1, 0, u->st>>>(u->sums, n0, u->rms);
   k_input_bf16<<<blocks_for(n0), 256, 0, u->st>>>(xbp, n0, u->rms, u->b_in0);
   u->launches += 3;
@@ -818,9 +914,9 @@ int forward_bf16(rihvr_unet* u, const float2* xbp, float2* x0, float scale) {
   if ((rc = conv_bf16(u, 2, u->b_a2)) || (rc = conv_bf16(u, 3, u->b_a3))) return rc;
   k_pool_bf16<<<blocks_for(n2 * 4), 256, 0, u->st>>>(u->b_a3, u->b_p2, u->lv[2], 32);
   if ((rc = conv_bf16(u, 4, u->b_a4)) || (rc = conv_bf16(u, 5, u->b_a5))) return rc;
-  k_up_concat_bf16<<<blocks_for(n1 * 12), 256, 0, u->st>>>(u->b_a5, 64, u->b_a3, 32, u->b_c2, u->lv[1]);
+  k_up_bf16<<<rows_of(u->lv[1]), 256, 0, u->st>>>(u->b_a5, 64, u->b_c2, u->lv[1]);
   if ((rc = conv_bf16(u, 6, u->b_a2)) || (rc = conv_bf16(u, 7, u->b_a7))) return rc;
-  k_up_concat_bf16<<<blocks_for(n0 * 6), 256, 0, u->st>>>(u->b_a7, 32, u->b_a1, 16, u->b_c1, u->lv[0]);
+  k_up_bf16<<<rows_of(u->lv[0]), 256, 0, u->st>>>(u->b_a7, 32, u->b_c1, u->lv[0]);
   if ((rc = conv_bf16(u, 8, u->b_a0))) return rc;
   TcHead hd;
   hd.w = u->w + u->head_off;
@@ -941,6 +1037,7 @@ int rihvr_unet_create(int depth, int height, int width, unsigned long long seed,
   A(&u->D2b, n2 * 64);
   A(&u->P2, n2 * 32);
   A(&u->rms, 1);
+  A(&u->head_parts, (size_t)18 * 8 * blocks_for(n0));
   if (rc == RIHVR_OK) rc = ualloc(u, &u->sums, 3);
   if (rc == RIHVR_OK) rc = ualloc(u, &u->tc_err, 1);
   if (rc == RIHVR_OK) rc = ualloc(u, &u->x0tmp, (size_t)n0);

@@ -7,7 +7,11 @@
 // operands, and all 27 taps read their shifted windows of that halo.  Its nine
 // warps take the nine (dz, dy) pairs, three dx taps each; the partial sums of
 // a warp's 3 taps x Cout x 16 stay in FP32 registers over all of the block's
-// bricks and reach memory as one atomic add each at the end.  Both operands
+// bricks and reach memory as one atomic add each at the end.  The tensor core's
+// own accumulation truncates, so a chain of MMAs ends after at most 16 steps
+// (256 voxels) in a rounded FP32 add to a second set of registers; at 64 output
+// channels, where these do not fit, a block takes two small bricks and ends.
+// (One chain over a block's bricks left the gradients 1.5e-5 off.)  Both operands
 // lie voxel by voxel, so the fragments of mma.sync m16n8k16 (M = output
 // channels, N = input channels, K = 16 voxels of an x-row) come through
 // ldmatrix.trans, without a transposed copy.
@@ -16,7 +20,7 @@
 // MMAs at 16 output channels).  The form before it gave every tap and slice a
 // grid of its own, which staged every voxel of X and dY 27 times through
 // scalar transposing stores and added its sums by atomics every 1024 voxels: the
-// gradients of a 32 x 128 x 128 volume took 16.2 ms with it, 2.8 ms with this one
+// gradients of a 32 x 128 x 128 volume took 16.2 ms with it, 2.3 ms with this one
 // (a 16 -> 16 layer at full size 53 us).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -91,13 +95,24 @@ __global__ void __launch_bounds__(kWgThreads)
   const int mr = lane & 7, m = lane >> 3;
   const int a_vox = mr + (m >> 1) * 8, a_chunk = m & 1;  // A: (voxels, co) quarters
   const int b_vox = mr + (m & 1) * 8, b_chunk = m >> 1;  // B: (voxels, ci) quarters
-  float acc[3][COT][2][4];
+  constexpr bool SUMS = COT <= 2;  // a second set of registers takes the chains' results
+  constexpr int ROWS = 16 * 16 / BX < BZ * BY ? 16 * 16 / BX : BZ * BY;  // x-rows of a chain
+  static_assert(BZ * BY % ROWS == 0, "whole chains");
+  float acc[3][COT][2][4], sum[SUMS ? 3 : 1][SUMS ? COT : 1][2][4];
+  auto each = [&](auto fn) {
 #pragma unroll
-  for (int t = 0; t < 3; ++t)
+    for (int t = 0; t < 3; ++t)
 #pragma unroll
-    for (int i = 0; i < COT; ++i)
+      for (int i = 0; i < COT; ++i)
 #pragma unroll
-      for (int j = 0; j < 2; ++j) acc[t][i][j][0] = acc[t][i][j][1] = acc[t][i][j][2] = acc[t][i][j][3] = 0.f;
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int h = 0; h < 4; ++h) fn(t, i, j, h);
+  };
+  each([&](int t, int i, int j, int h) {
+    acc[t][i][j][h] = 0.f;
+    if constexpr (SUMS) sum[t][i][j][h] = 0.f;
+  });
 #pragma unroll 1
   for (int b = blockIdx.x; b < bricks; b += gridDim.x) {
     const int x0 = (b % nbx) * BX, y0 = ((b / nbx) % nby) * BY, z0 = (b / (nbx * nby)) * BZ;
@@ -119,6 +134,13 @@ __global__ void __launch_bounds__(kWgThreads)
     __syncthreads();
 #pragma unroll 1
     for (int row = 0; row < BZ * BY; ++row) {
+      if constexpr (SUMS) {
+        if (row % ROWS == 0)
+          each([&](int t, int i, int j, int h) {
+            sum[t][i][j][h] += acc[t][i][j][h];
+            acc[t][i][j][h] = 0.f;
+          });
+      }
       const int rz = row / BY, ry = row % BY;
       const int hrow = ((rz + dz) * Sh::HY + ry + dy) * Sh::HX;  // halo voxel left of the row (dx = 0)
 #pragma unroll
@@ -141,6 +163,7 @@ __global__ void __launch_bounds__(kWgThreads)
     }
     __syncthreads();
   }
+  if constexpr (SUMS) each([&](int t, int i, int j, int h) { acc[t][i][j][h] += sum[t][i][j][h]; });
   const int g = lane >> 2, t4 = lane & 3;
 #pragma unroll
   for (int t = 0; t < 3; ++t) {
@@ -168,7 +191,9 @@ cudaError_t wgrad_launch(const float* X, int Cin, const float* dY, float* dW, in
   const long long bricks = (long long)((W + BX - 1) / BX) * ((H + BY - 1) / BY) * ((D + BZ - 1) / BZ);
   if (bricks > 0x7fffffffLL) return cudaErrorInvalidValue;
   const int slices = Cin / 16;
-  const int gx = (int)std::min<long long>(bricks, std::max(1, blocks_max / slices));
+  // a block's walk over the bricks, or, without the second registers, two of them
+  const int gx = COT <= 2 ? (int)std::min<long long>(bricks, std::max(1, blocks_max / slices))
+                          : (int)((bricks + 1) / 2);
   k_wgrad<COT, BZ, BY, BX><<<dim3(gx, slices), kWgThreads, Sh::SMEM, st>>>(X, Cin, dY, dW, D, H, W, (int)bricks);
   return cudaGetLastError();
 }

@@ -342,7 +342,9 @@ constexpr size_t tcb_smem() {
 }
 
 template <int CN, bool HEAD>
-__global__ void __launch_bounds__(kTcThreads) k_conv3_tc_bf16(const __grid_constant__ CUtensorMap xmap, int Cin,
+__global__ void __launch_bounds__(kTcThreads) k_conv3_tc_bf16(const __grid_constant__ CUtensorMap xmap,
+                                                              const __grid_constant__ CUtensorMap skipmap,
+                                                              int CinA, int Cin,
                                                               const __nv_bfloat16* __restrict__ Wp,
                                                               const float* __restrict__ bias,
                                                               __nv_bfloat16* __restrict__ Y, int D, int H, int W,
@@ -395,8 +397,11 @@ __global__ void __launch_bounds__(kTcThreads) k_conv3_tc_bf16(const __grid_const
         if (!ok) break;
       }
       mbar_expect_tx(bar_full, 2u * kTcBoxBytes + BBYTES);
-      tma_load_4d(a0, &xmap, 16 * s, x0 - 1, y0 - 1, z0 - 1, bar_full);
-      tma_load_4d(a0 + kTcPlaneBytes, &xmap, 16 * s + 8, x0 - 1, y0 - 1, z0 - 1, bar_full);
+      const bool skip = 16 * s >= CinA;
+      const CUtensorMap* const map = skip ? &skipmap : &xmap;
+      const int ch = 16 * s - (skip ? CinA : 0);
+      tma_load_4d(a0, map, ch, x0 - 1, y0 - 1, z0 - 1, bar_full);
+      tma_load_4d(a0 + kTcPlaneBytes, map, ch + 8, x0 - 1, y0 - 1, z0 - 1, bar_full);
       bulk_load(b0, Wp + (size_t)s * (BBYTES / 2), BBYTES, bar_full);
       ok = mbar_wait(bar_full, pf);
       pf ^= 1u;
@@ -698,7 +703,7 @@ EncodeTiledFn encode_tiled() {
 }
 
 template <int CN, bool HEAD>
-cudaError_t tcb_launch(const TcMap& m, int Cin, const __nv_bfloat16* Wp, const float* bias, __nv_bfloat16* Y, int D,
+cudaError_t tcb_launch(const TcMap& m, const TcMap& ms, int CinA, int Cin, const __nv_bfloat16* Wp, const float* bias, __nv_bfloat16* Y, int D,
                        int H, int W, const TcHead& hd, int* err, cudaStream_t st) {
   constexpr size_t smem = tcb_smem<CN>();
   static bool opted = false;
@@ -708,11 +713,12 @@ cudaError_t tcb_launch(const TcMap& m, int Cin, const __nv_bfloat16* Wp, const f
     if (e != cudaSuccess) return e;
     opted = true;
   }
-  CUtensorMap map;
+  CUtensorMap map, smap;
   static_assert(sizeof(map) == sizeof(m.bytes), "tensor map size");
   std::memcpy(&map, m.bytes, sizeof(map));
+  std::memcpy(&smap, CinA < Cin ? ms.bytes : m.bytes, sizeof(smap));
   const unsigned blocks = (unsigned)((W / kTcX) * ((H + kTcYT - 1) / kTcYT) * D);
-  k_conv3_tc_bf16<CN, HEAD><<<blocks, kTcThreads, smem, st>>>(map, Cin, Wp, bias, Y, D, H, W, hd, err);
+  k_conv3_tc_bf16<CN, HEAD><<<blocks, kTcThreads, smem, st>>>(map, smap, CinA, Cin, Wp, bias, Y, D, H, W, hd, err);
   return cudaGetLastError();
 }
 
@@ -836,19 +842,19 @@ cudaError_t tc_weights(const float* w, int Cout, int Cin, __nv_bfloat16* wp, cud
   return cudaGetLastError();
 }
 
-cudaError_t conv3_tc_bf16(const TcMap& xmap, int Cin, const __nv_bfloat16* Wp, const float* bias, int Cout,
-                          __nv_bfloat16* Y, int D, int H, int W, const TcHead* head, int* err, cudaStream_t st) {
-  if (!conv3_tc_bf16_supported(D, H, W, Cin, Cout)) return cudaErrorInvalidValue;
+cudaError_t conv3_tc_bf16(const TcMap& xmap, const TcMap& skipmap, int CinA, int Cin, const __nv_bfloat16* Wp,
+                          const float* bias, int Cout, __nv_bfloat16* Y, int D, int H, int W, const TcHead* head, int* err, cudaStream_t st) {
+  if (!conv3_tc_bf16_supported(D, H, W, Cin, Cout) || CinA % 16 != 0 || CinA > Cin) return cudaErrorInvalidValue;
   const TcHead hd = head ? *head : TcHead{};
   if (head) {
     if (Cout != 16) return cudaErrorInvalidValue;
-    return tcb_launch<16, true>(xmap, Cin, Wp, bias, Y, D, H, W, hd, err, st);
+    return tcb_launch<16, true>(xmap, skipmap, CinA, Cin, Wp, bias, Y, D, H, W, hd, err, st);
   }
   switch (Cout) {
-    case 16: return tcb_launch<16, false>(xmap, Cin, Wp, bias, Y, D, H, W, hd, err, st);
-    case 32: return tcb_launch<32, false>(xmap, Cin, Wp, bias, Y, D, H, W, hd, err, st);
-    case 48: return tcb_launch<48, false>(xmap, Cin, Wp, bias, Y, D, H, W, hd, err, st);
-    default: return tcb_launch<64, false>(xmap, Cin, Wp, bias, Y, D, H, W, hd, err, st);
+    case 16: return tcb_launch<16, false>(xmap, skipmap, CinA, Cin, Wp, bias, Y, D, H, W, hd, err, st);
+    case 32: return tcb_launch<32, false>(xmap, skipmap, CinA, Cin, Wp, bias, Y, D, H, W, hd, err, st);
+    case 48: return tcb_launch<48, false>(xmap, skipmap, CinA, Cin, Wp, bias, Y, D, H, W, hd, err, st);
+    default: return tcb_launch<64, false>(xmap, skipmap, CinA, Cin, Wp, bias, Y, D, H, W, hd, err, st);
   }
 }
 

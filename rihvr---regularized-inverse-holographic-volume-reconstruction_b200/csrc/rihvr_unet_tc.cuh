@@ -35,7 +35,9 @@ bool tc_map_encode(TcMap* m, const __nv_bfloat16* X, int C, int D, int H, int W)
 bool conv3_tc_bf16_supported(int D, int H, int W, int Cin, int Cout);
 size_t tc_weights_elems(int Cout, int Cin);
 cudaError_t tc_weights(const float* w, int Cout, int Cin, __nv_bfloat16* wp, cudaStream_t st);
-cudaError_t conv3_tc_bf16(const TcMap& xmap, int Cin, const __nv_bfloat16* Wp, const float* bias, int Cout,
+// The first CinA of the Cin input channels are xmap's, the others skipmap's
+// (a second tensor of the same volume; CinA = Cin: none).
+cudaError_t conv3_tc_bf16(const TcMap& xmap, const TcMap& skipmap, int CinA, int Cin, const __nv_bfloat16* Wp, const float* bias, int Cout,
                           __nv_bfloat16* Y, int D, int H, int W, const TcHead* head, int* err, cudaStream_t st);
 
 // The z-walking form of the same convolution (16 input channels, 16 or 32
