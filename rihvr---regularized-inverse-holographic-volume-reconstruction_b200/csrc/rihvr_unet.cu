@@ -877,7 +877,7 @@ int bf16_prepare(rihvr_unet* u) {
       return RIHVR_OK;
     }
     u->zwalk[i] = use_zwalk() && tcz_supported(v.W, L.cin, L.cout) &&
-                  tc_zmap_encode(&u->zmaps[i], in[i], L.cin, v.D, v.H, v.W, tcz_rows(L.cin) + 2);
+                  tc_zmap_encode(&u->zmaps[i], in[i], L.cin, v.D, v.H, v.W, tcz_rows(L.cout) + 2);
   }
   u->bf_ready = true;
   return RIHVR_OK;

@@ -484,54 +484,69 @@ __global__ void __launch_bounds__(kTcThreads) k_conv3_tc_bf16(const __grid_const
 
 // ---------------------------------------------------------------------------
 // z-walking form of the inference convolution, for layers with 16 input
-// channels (the template also takes more slices, NS).  A block keeps one
-// (x-tile of 128 voxels, y-tile of YT rows) column and walks a range of z.
-// Shared memory holds a ring of 3 input slabs (one z-plane each: YT + 2 rows x
-// 130 voxels, every slice in two 8-channel planes, the layout the descriptors
-// read), so each input plane is loaded once per block instead of three times,
-// and the weights of all slices, loaded once per block.  Per output plane z:
-//   thread 0 waits for slab z+1, issues the 27 x YT x slices MMAs into the
-//   tensor-memory accumulator and commits them; once they are done it reuses
-//   slab z-1's slot for slab z+2 (one TMA box per slice and half, completing on
-//   that slot's mbarrier) while all threads drain the accumulator (bias, ReLU,
-//   BF16 store, or the head).  The TMA copy overlaps the epilogue, and a
-//   second block on the SM (16 channels: 89 KB a block) fills the tensor pipe
-//   while this one drains.
+// channels.  A block keeps one (x-tile of 128 voxels, y-tile of YT rows) column
+// and walks a range of z, one input slab (a z-plane of YT + 2 rows x 130 voxels
+// in two 8-channel planes, the layout the descriptors read) at a time.  An
+// input voxel contributes to the output planes below, at and above it, so the
+// three dz taps of a (dy, dx) go into ONE MMA of N = 3 CN: its accumulators are
+// the three output planes in work, side by side in tensor memory, and its B
+// operand the three taps' weights in the order of those planes.  Output plane o
+// lies in slot o mod 3, so that order is one of the three rotations of
+// (dz = 1, 0, -1); the weights are stored as dz = 1, 0, -1, 1, 0 for every
+// (dy, dx) and a rotation is an offset into them.  A slab takes 9 x YT MMAs:
+// with N = CN, 27 x YT were bound by their reads of A from shared memory, which
+// do not depend on N (16 -> 16 channels on 100 x 512 x 512: 1.21 ms then, 0.72 ms
+// so; 16 -> 32 on 50 x 256 x 256: 255 and 173 us).
+// An output plane adds its taps in the same order (dz, dy, dx) as they did.
+//   Per slab z thread 0 waits for it, issues and commits the MMAs and, once they
+// are done, reuses its slot for slab z + 3 (one TMA box per half, completing on
+// that slot's mbarrier); all threads then drain output plane z - 1 (bias, ReLU,
+// BF16 store, or the head) and clear its accumulator for plane z + 2.  The
+// second block on the SM fills the tensor pipe meanwhile.
 // Every wait is bounded; a wait that runs out sets *err, the block lets its
 // copies and MMAs in flight finish (bounded) and leaves.
 // ---------------------------------------------------------------------------
-template <int YT, int NS>  // x-rows a block, 16-channel slices
+template <int CN>
 struct TczShape {
+  static constexpr int YT = CN == 16 ? 4 : 2;                       // x-rows a block: 192 accumulator columns
   static constexpr int HY = YT + 2;
   static constexpr uint32_t BOX = 16u * kTcHX * HY;                 // one 8-channel plane of a slab
   static constexpr uint32_t PLANE = (BOX + 127u) / 128u * 128u;     // planes 128 bytes apart
-  static constexpr uint32_t SLAB = 2u * NS * PLANE;
-  static constexpr int R = 3;                                        // slabs in the ring
+  static constexpr uint32_t SLAB = 2u * PLANE;
+  static constexpr int R = 3;                                       // slabs in the ring
+  static constexpr uint32_t NCOLS = 256;                            // of YT x 3 x CN = 192
+  static constexpr uint32_t BHALF = 9u * 5u * CN * 16u;             // weights of one 8-channel half
 };
 
-template <int CN, int YT, int NS>
+template <int CN>
 constexpr size_t tcz_smem() {
-  using S = TczShape<YT, NS>;
-  return 1024 + (size_t)S::R * S::SLAB + (size_t)NS * 2 * 27 * CN * 16 + 64;
+  using S = TczShape<CN>;
+  return 1024 + (size_t)S::R * S::SLAB + 2 * (size_t)S::BHALF + 64;
 }
 
-template <int CN, bool HEAD, int YT, int NS>
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr),
+      "r"(0u)
+      : "memory");
+}
+
+template <int CN, bool HEAD>
 __global__ void __launch_bounds__(kTcThreads) k_conv3_tcz(const __grid_constant__ CUtensorMap zmap,
                                                           const __nv_bfloat16* __restrict__ Wp,
                                                           const float* __restrict__ bias,
                                                           __nv_bfloat16* __restrict__ Y, int D, int H, int W,
                                                           int zper, TcHead hd, int* __restrict__ err) {
-  static_assert(CN % 16 == 0 && CN >= 16 && CN <= 64, "N of the MMA");
+  static_assert(CN == 16 || CN == 32, "output channels");
   static_assert(!HEAD || CN == 16, "the head takes 16 channels");
-  using S = TczShape<YT, NS>;
-  constexpr uint32_t NCOLS = YT * CN <= 32 ? 32u : YT * CN <= 64 ? 64u : YT * CN <= 128 ? 128u : 256u;
-  constexpr uint32_t BBYTES = 2u * 27u * CN * 16u;  // one slice's weights
+  using S = TczShape<CN>;
+  constexpr int YT = S::YT;
   extern __shared__ unsigned char tzraw[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tzraw) + 1023) & ~uintptr_t(1023));
-  unsigned char* slabs = base;                          // [R][NS][2 planes] of PLANE bytes
-  unsigned char* B0 = slabs + S::R * S::SLAB;           // [NS][2][27 * CN] x 16 B
-  uint64_t* bars = reinterpret_cast<uint64_t*>(B0 + NS * BBYTES);  // [0..2] slabs, [3] weights, [4] MMAs
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 5);
+  unsigned char* slabs = base;                          // [R][2 planes] of PLANE bytes
+  unsigned char* B0 = slabs + S::R * S::SLAB;           // [2 halves][9][5][CN] x 16 B
+  uint64_t* bars = reinterpret_cast<uint64_t*>(B0 + 2 * S::BHALF);  // [0..2] slabs, [3] MMAs
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 4);
   int* s_ok = reinterpret_cast<int*>(tslot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nbx = W / kTcX, nby = (H + YT - 1) / YT;
@@ -541,84 +556,80 @@ __global__ void __launch_bounds__(kTcThreads) k_conv3_tcz(const __grid_constant_
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(tslot)),
-                 "r"(NCOLS)
+                 "r"(S::NCOLS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (tid == 0) {
-    for (int i = 0; i < 5; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(saddr(bars + i)) : "memory");
+    for (int i = 0; i < 4; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(saddr(bars + i)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     *s_ok = 1;
   }
+  // weights: row (half, dy dx, j, co) is tap dz = 1, 0, -1, 1, 0 for j = 0..4 of the layer's [half][27][CN] rows
+  for (int e = tid; e < 2 * 9 * 5 * CN; e += kTcThreads) {
+    const int co = e % CN, j = e / CN % 5, t9 = e / (5 * CN) % 9, half = e / (45 * CN);
+    const int kz = (2 * j + 2) % 3;  // 2, 1, 0, 2, 1
+    reinterpret_cast<uint4*>(B0)[e] = __ldg(reinterpret_cast<const uint4*>(Wp) + (half * 27 + kz * 9 + t9) * CN + co);
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes -> tensor-core reads
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tbase = *tslot;
-  const uint32_t idesc = instr_desc(CN);
+  const uint32_t twarp = tbase + ((uint32_t)(warp * 32) << 16);  // this warp's lanes
+  const uint32_t idesc = instr_desc(3 * CN);
   const uint32_t s0 = saddr(slabs), b0 = saddr(B0);
   uint32_t phase[S::R] = {0u, 0u, 0u};  // thread 0: parity of each slot's next completion
   bool busy[S::R] = {false, false, false};  // a copy into the slot not yet awaited
   uint32_t pm = 0;                      // parity of the MMA barrier
-  bool mma_busy = false, w_busy = false;
+  bool mma_busy = false;
   bool ok = true;
-  // slot of the slab of plane z: the ring starts with plane zb - 1 in slot 0
-  auto slot_of = [&](int z) { return (uint32_t)((z - zb + 1) % S::R); };
-  auto load_slab = [&](int z) {  // thread 0
-    const uint32_t sl = slot_of(z);
+  auto load_slab = [&](int z, uint32_t sl) {  // thread 0
     const uint32_t bar = saddr(bars + sl);
     busy[sl] = true;
-    mbar_expect_tx(bar, 2u * NS * S::BOX);
+    mbar_expect_tx(bar, 2u * S::BOX);
 #pragma unroll
-    for (int sc = 0; sc < NS; ++sc)
-#pragma unroll
-      for (int p = 0; p < 2; ++p)
-        tma_load_4d(s0 + sl * S::SLAB + (uint32_t)(sc * 2 + p) * S::PLANE, &zmap, 16 * sc + 8 * p, x0 - 1, y0 - 1,
-                    z, bar);
+    for (int p = 0; p < 2; ++p)
+      tma_load_4d(s0 + sl * S::SLAB + (uint32_t)p * S::PLANE, &zmap, 8 * p, x0 - 1, y0 - 1, z, bar);
   };
-  if (tid == 0 && zb < ze) {
-    mbar_expect_tx(saddr(bars + 3), NS * BBYTES);
-    bulk_load(b0, Wp, NS * BBYTES, saddr(bars + 3));
-    w_busy = true;
-    for (int z = zb - 1; z <= zb + 1; ++z) load_slab(z);  // planes outside the volume read as zeros
-    ok = mbar_wait(saddr(bars + 3), 0);
-    w_busy = !ok;
-    for (int z = zb - 1; z <= zb && ok; ++z) {
-      ok = mbar_wait(saddr(bars + slot_of(z)), phase[slot_of(z)]);
-      if (ok) {
-        phase[slot_of(z)] ^= 1u;
-        busy[slot_of(z)] = false;
-      }
-    }
-  }
-  for (int z = zb; z < ze; ++z) {
+  // the ring starts with plane zb - 1 in slot 0; planes outside the volume read as zeros
+  if (tid == 0 && zb < ze)
+    for (int i = 0; i < S::R && zb - 1 + i <= ze; ++i) load_slab(zb - 1 + i, (uint32_t)i);
+#pragma unroll
+  for (int i = 0; i < YT * 3 * CN / 16; ++i) tmem_zero16(twarp + (uint32_t)(16 * i));
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  uint32_t r3 = 0;  // (z - zb + 1) mod 3: slab z's slot in the ring and output plane z's accumulator
+  for (int z = zb - 1; z <= ze; ++z) {
+    const uint32_t below = r3 == 0 ? 2u : r3 - 1u;  // output plane z - 1's accumulator
     if (tid == 0) {
-      if (ok) {  // slab z+1, the last one this plane reads
-        ok = mbar_wait(saddr(bars + slot_of(z + 1)), phase[slot_of(z + 1)]);
+      if (ok) {
+        ok = mbar_wait(saddr(bars + r3), phase[r3]);
         if (ok) {
-          phase[slot_of(z + 1)] ^= 1u;
-          busy[slot_of(z + 1)] = false;
+          phase[r3] ^= 1u;
+          busy[r3] = false;
         }
       }
       if (ok) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint64_t ad = smem_desc(s0 + r3 * S::SLAB, S::PLANE, 128);
+        // slots hold planes with dz (1, 0, -1) from slot `below` on
+        const uint64_t bd = smem_desc(b0, S::BHALF, 128) + (uint64_t)((3u - below) % 3u * CN);
 #pragma unroll
-        for (int sc = 0; sc < NS; ++sc) {
-          uint64_t ad[3];
+        for (int k = 0; k < 9; ++k)
 #pragma unroll
-          for (int d = 0; d < 3; ++d)
-            ad[d] = smem_desc(s0 + slot_of(z + d - 1) * S::SLAB + (uint32_t)(sc * 2) * S::PLANE, S::PLANE, 128);
-          const uint64_t bd = smem_desc(b0 + (uint32_t)sc * BBYTES, 27 * CN * 16, 128);
-          issue_slice<CN, YT, S::HY, false>(tbase, ad, bd, idesc, sc > 0);
-        }
-        mma_commit(saddr(bars + 4));
+          for (int m = 0; m < YT; ++m)
+            mma_bf16_ss(tbase + (uint32_t)(m * 3 * CN), ad + (uint64_t)((m + k / 3) * kTcHX + k % 3),
+                        bd + (uint64_t)(k * 5 * CN), idesc, 1u);
+        mma_commit(saddr(bars + 3));
         mma_busy = true;
-        ok = mbar_wait(saddr(bars + 4), pm);
+        ok = mbar_wait(saddr(bars + 3), pm);
         if (ok) {
           pm ^= 1u;
           mma_busy = false;
         }
-        // slab z-1 is no longer read: its slot takes slab z+2 for the next plane
-        if (ok && z + 1 < ze) load_slab(z + 2);
+        if (ok && z + S::R <= ze) load_slab(z + S::R, r3);
       }
       if (!ok) *s_ok = 0;
     }
@@ -628,61 +639,67 @@ __global__ void __launch_bounds__(kTcThreads) k_conv3_tcz(const __grid_constant_
     const int xx = x0 + warp * 32 + lane;
 #pragma unroll 1
     for (int m = 0; m < YT; ++m) {
+      const uint32_t acc = twarp + (uint32_t)(m * 3 * CN) + below * CN;
       const int yy = y0 + m;
-      const long long vox = ((long long)z * H + yy) * W + xx;
+      const long long vox = ((long long)(z - 1) * H + yy) * W + xx;
       float zsum = 0.f;
       if constexpr (HEAD) zsum = hd.w[16];
+      if (z > zb) {
 #pragma unroll
-      for (int c16 = 0; c16 < CN / 16; ++c16) {
-        float v[16];
-        tmem_ld16(tbase + ((uint32_t)(warp * 32) << 16) + (uint32_t)(m * CN + c16 * 16), v);
+        for (int c16 = 0; c16 < CN / 16; ++c16) {
+          float v[16];
+          tmem_ld16(acc + (uint32_t)(c16 * 16), v);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = fmaxf(v[j] + bias[c16 * 16 + j], 0.f);
+          for (int j = 0; j < 16; ++j) v[j] = fmaxf(v[j] + bias[c16 * 16 + j], 0.f);
+          if constexpr (HEAD) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) zsum += hd.w[j] * v[j];
+          } else if (yy < H) {
+            uint4 o0, o1;
+            o0.x = pack2(v[0], v[1]);
+            o0.y = pack2(v[2], v[3]);
+            o0.z = pack2(v[4], v[5]);
+            o0.w = pack2(v[6], v[7]);
+            o1.x = pack2(v[8], v[9]);
+            o1.y = pack2(v[10], v[11]);
+            o1.z = pack2(v[12], v[13]);
+            o1.w = pack2(v[14], v[15]);
+            uint4* dst = reinterpret_cast<uint4*>(Y + vox * CN + c16 * 16);
+            dst[0] = o0;
+            dst[1] = o1;
+          }
+        }
         if constexpr (HEAD) {
+          if (yy < H) {
+            const float g = 1.f / (1.f + expf(-zsum));
+            const float alpha = hd.w[17] * hd.scale;
+            const float2 a = hd.xbp[vox];
+            hd.x0[vox] = make_float2(g * alpha * a.x, g * alpha * a.y);
+          }
+        }
+      }
 #pragma unroll
-          for (int j = 0; j < 16; ++j) zsum += hd.w[j] * v[j];
-        } else if (yy < H) {
-          uint4 o0, o1;
-          o0.x = pack2(v[0], v[1]);
-          o0.y = pack2(v[2], v[3]);
-          o0.z = pack2(v[4], v[5]);
-          o0.w = pack2(v[6], v[7]);
-          o1.x = pack2(v[8], v[9]);
-          o1.y = pack2(v[10], v[11]);
-          o1.z = pack2(v[12], v[13]);
-          o1.w = pack2(v[14], v[15]);
-          uint4* dst = reinterpret_cast<uint4*>(Y + vox * CN + c16 * 16);
-          dst[0] = o0;
-          dst[1] = o1;
-        }
-      }
-      if constexpr (HEAD) {
-        if (yy < H) {
-          const float g = 1.f / (1.f + expf(-zsum));
-          const float alpha = hd.w[17] * hd.scale;
-          const float2 a = hd.xbp[vox];
-          hd.x0[vox] = make_float2(g * alpha * a.x, g * alpha * a.y);
-        }
-      }
+      for (int c16 = 0; c16 < CN / 16; ++c16) tmem_zero16(acc + (uint32_t)(c16 * 16));
     }
-    // every thread's accumulator reads come before the next plane's MMAs
+    // every thread's accumulator reads and clears come before the next slab's MMAs
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    r3 = r3 == 2 ? 0u : r3 + 1u;
   }
   if (tid == 0 && !ok) {
     atomicExch(err, 1);
     // a last bounded wait for the copies and MMAs still in flight before the
     // shared and tensor memory are released
-    if (mma_busy) mbar_wait(saddr(bars + 4), pm);
+    if (mma_busy) mbar_wait(saddr(bars + 3), pm);
     for (int i = 0; i < S::R; ++i)
       if (busy[i]) mbar_wait(saddr(bars + i), phase[i]);
-    if (w_busy) mbar_wait(saddr(bars + 3), 0);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(NCOLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(S::NCOLS) : "memory");
   }
 }
 
@@ -753,7 +770,7 @@ bool tc_map_encode(TcMap* m, const __nv_bfloat16* X, int C, int D, int H, int W)
 }
 
 // x-rows a block of the z-walking form takes
-int tcz_rows(int) { return 4; }
+int tcz_rows(int Cout) { return Cout == 16 ? TczShape<16>::YT : TczShape<32>::YT; }
 
 bool tc_zmap_encode(TcMap* m, const __nv_bfloat16* X, int C, int D, int H, int W, int rows) {
   const EncodeTiledFn enc = encode_tiled();
@@ -772,7 +789,9 @@ bool tc_zmap_encode(TcMap* m, const __nv_bfloat16* X, int C, int D, int H, int W
   return true;
 }
 
-// 16 input channels only: with three slices (48 channels) the ring and the
+// 16 input channels only: 48 channels would add their three slices plane by plane
+// instead of one after another (other roundings), and walking z in the old order
+// the ring and the
 // weights fill the shared memory of one block an SM, and that layer measured
 // slower walking z (a block's loads, MMAs and epilogue then have nothing to
 // overlap with) than in the per-tile kernel.
@@ -781,40 +800,48 @@ bool tcz_supported(int W, int Cin, int Cout) {
 }
 
 namespace {
-template <int CN, bool HEAD, int YT, int NS>
+template <int CN, bool HEAD>
 cudaError_t tcz_launch(const TcMap& m, const __nv_bfloat16* Wp, const float* bias, __nv_bfloat16* Y, int D, int H,
                        int W, const TcHead& hd, int* err, cudaStream_t st) {
-  constexpr size_t smem = tcz_smem<CN, YT, NS>();
+  constexpr int YT = TczShape<CN>::YT;
+  constexpr size_t smem = tcz_smem<CN>();
+  const auto kern = k_conv3_tcz<CN, HEAD>;
   static bool opted = false;
   if (!opted) {
-    const cudaError_t e = cudaFuncSetAttribute(k_conv3_tcz<CN, HEAD, YT, NS>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     opted = true;
   }
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_conv3_tcz<CN, HEAD, YT, NS>, kTcThreads, smem) !=
-          cudaSuccess ||
-      per_sm < 1) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTcThreads, smem) != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
     per_sm = 1;
   }
+  per_sm = std::min(per_sm, (int)(512 / TczShape<CN>::NCOLS));  // tensor memory
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) !=
                                                  cudaSuccess) {
     cudaGetLastError();
     sms = 148;
   }
-  // z-ranges per (x, y) column: about four waves of blocks in all
+  // z-ranges per (x, y) column: whole waves of blocks against the two slabs each range reads beyond its own
   const long long xy = (long long)(W / kTcX) * ((H + YT - 1) / YT);
-  const long long target = 4LL * sms * per_sm;
-  const int zsplit = (int)std::max(1LL, std::min<long long>(D, (target + xy - 1) / xy));
-  const int zper = (D + zsplit - 1) / zsplit;
+  int zper = D;
+  double best = 1e300;
+  for (int n = 1; n <= D && n <= 64; ++n) {
+    const int len = (D + n - 1) / n;
+    const double waves = std::ceil((double)xy * ((D + len - 1) / len) / ((double)sms * per_sm));
+    const double cost = waves * (len + 3);
+    if (cost < best * 0.999) {
+      best = cost;
+      zper = len;
+    }
+  }
   const long long blocks = xy * ((D + zper - 1) / zper);
   if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   CUtensorMap map;
   std::memcpy(&map, m.bytes, sizeof(map));
-  k_conv3_tcz<CN, HEAD, YT, NS><<<(unsigned)blocks, kTcThreads, smem, st>>>(map, Wp, bias, Y, D, H, W, zper, hd, err);
+  kern<<<(unsigned)blocks, kTcThreads, smem, st>>>(map, Wp, bias, Y, D, H, W, zper, hd, err);
   return cudaGetLastError();
 }
 }  // namespace
@@ -823,9 +850,9 @@ cudaError_t conv3_tcz(const TcMap& zmap, int Cin, const __nv_bfloat16* Wp, const
                       __nv_bfloat16* Y, int D, int H, int W, const TcHead* head, int* err, cudaStream_t st) {
   if (!tcz_supported(W, Cin, Cout) || (head && Cout != 16)) return cudaErrorInvalidValue;
   const TcHead hd = head ? *head : TcHead{};
-  if (head) return tcz_launch<16, true, 4, 1>(zmap, Wp, bias, Y, D, H, W, hd, err, st);
-  return Cout == 16 ? tcz_launch<16, false, 4, 1>(zmap, Wp, bias, Y, D, H, W, hd, err, st)
-                    : tcz_launch<32, false, 4, 1>(zmap, Wp, bias, Y, D, H, W, hd, err, st);
+  if (head) return tcz_launch<16, true>(zmap, Wp, bias, Y, D, H, W, hd, err, st);
+  return Cout == 16 ? tcz_launch<16, false>(zmap, Wp, bias, Y, D, H, W, hd, err, st)
+                    : tcz_launch<32, false>(zmap, Wp, bias, Y, D, H, W, hd, err, st);
 }
 
 bool conv3_tc_bf16_supported(int D, int H, int W, int Cin, int Cout) {
