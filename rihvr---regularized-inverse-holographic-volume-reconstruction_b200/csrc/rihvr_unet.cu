@@ -496,8 +496,8 @@ __global__ void k_head_back(const float* __restrict__ Hh, const float* __restric
 // dw[c] += the warps' sums, one block a sum, added one after another in warp
 // order by one thread.  An empty volume's voxels all add the same value, and a
 // chain rounds every such addition alike (2e-5 of the largest sum at
-// 32 x 128 x 128, against a tree); this is the chain that an atomic add a warp makes, which had taken
-// nine tenths of the kernel above (315 us; 54 us without it), in
+// 32 x 128 x 128, against a tree); this is the chain that an atomic add a warp
+// makes, which had taken most of the kernel above (315 us; 54 us without it), in
 // 47 us.
 __global__ void k_head_sums(const float* __restrict__ parts, int nw, float* __restrict__ dw) {
   constexpr int CH = 2048;  // values staged at a time; zeros past the end do not change a sum
@@ -706,6 +706,7 @@ struct rihvr_unet {
   TcMap skip_maps[kNumConv] = {};  // the skip tensor of a decoder's first layer
   int cin_a[kNumConv] = {};        // input channels of `maps`; the others are the skip tensor's
   TcMap zmaps[kNumConv];  // the z-walking form's maps, where a layer takes it
+  TcMap skip_zmaps[kNumConv] = {};
   bool zwalk[kNumConv] = {};
   float* head_parts = nullptr;  // warps' sums of the head's gradient
   double* sums = nullptr;   // [0] sum |xbp|^2, [1] sum |x*|^2, [2] loss
@@ -876,8 +877,10 @@ int bf16_prepare(rihvr_unet* u) {
       u->bf_failed = true;
       return RIHVR_OK;
     }
+    const int rows = tcz_rows(L.cin, L.cout) + 2;
     u->zwalk[i] = use_zwalk() && tcz_supported(v.W, L.cin, L.cout) &&
-                  tc_zmap_encode(&u->zmaps[i], in[i], L.cin, v.D, v.H, v.W, tcz_rows(L.cout) + 2);
+                  tc_zmap_encode(&u->zmaps[i], in[i], u->cin_a[i], v.D, v.H, v.W, rows) &&
+                  (!cskip || tc_zmap_encode(&u->skip_zmaps[i], i == 6 ? u->b_a3 : u->b_a1, cskip, v.D, v.H, v.W, rows));
   }
   u->bf_ready = true;
   return RIHVR_OK;
@@ -887,11 +890,11 @@ int conv_bf16(rihvr_unet* u, int li, __nv_bfloat16* Y, const TcHead* head = null
   const Conv& L = u->layers[li];
   const Vol v = u->lv[L.level];
   if (u->zwalk[li])
-    UCK(conv3_tcz(u->zmaps[li], L.cin, u->wtc + u->wtc_off[li], u->w + L.b_off, L.cout, Y, v.D, v.H, v.W, head,
-                  u->tc_err, u->st));
+    UCK(conv3_tcz(u->zmaps[li], u->skip_zmaps[li], u->cin_a[li], L.cin, u->wtc + u->wtc_off[li], u->w + L.b_off,
+                  L.cout, Y, v.D, v.H, v.W, head, u->tc_err, u->st));
   else
-    UCK(conv3_tc_bf16(u->maps[li], u->skip_maps[li], u->cin_a[li], L.cin, u->wtc + u->wtc_off[li], u->w + L.b_off, L.cout, Y, v.D, v.H, v.W, head,
-                      u->tc_err, u->st));
+    UCK(conv3_tc_bf16(u->maps[li], u->skip_maps[li], u->cin_a[li], L.cin, u->wtc + u->wtc_off[li], u->w + L.b_off,
+                      L.cout, Y, v.D, v.H, v.W, head, u->tc_err, u->st));
   ++u->launches;
   return RIHVR_OK;
 }

@@ -483,45 +483,60 @@ __global__ void __launch_bounds__(kTcThreads) k_conv3_tc_bf16(const __grid_const
 }
 
 // ---------------------------------------------------------------------------
-// z-walking form of the inference convolution, for layers with 16 input
-// channels.  A block keeps one (x-tile of 128 voxels, y-tile of YT rows) column
-// and walks a range of z, one input slab (a z-plane of YT + 2 rows x 130 voxels
-// in two 8-channel planes, the layout the descriptors read) at a time.  An
-// input voxel contributes to the output planes below, at and above it, so the
-// three dz taps of a (dy, dx) go into ONE MMA of N = 3 CN: its accumulators are
-// the three output planes in work, side by side in tensor memory, and its B
-// operand the three taps' weights in the order of those planes.  Output plane o
-// lies in slot o mod 3, so that order is one of the three rotations of
-// (dz = 1, 0, -1); the weights are stored as dz = 1, 0, -1, 1, 0 for every
-// (dy, dx) and a rotation is an offset into them.  A slab takes 9 x YT MMAs:
-// with N = CN, 27 x YT were bound by their reads of A from shared memory, which
-// do not depend on N (16 -> 16 channels on 100 x 512 x 512: 1.21 ms then, 0.72 ms
-// so; 16 -> 32 on 50 x 256 x 256: 255 and 173 us).
-// An output plane adds its taps in the same order (dz, dy, dx) as they did.
-//   Per slab z thread 0 waits for it, issues and commits the MMAs and, once they
-// are done, reuses its slot for slab z + 3 (one TMA box per half, completing on
-// that slot's mbarrier); all threads then drain output plane z - 1 (bias, ReLU,
-// BF16 store, or the head) and clear its accumulator for plane z + 2.  The
-// second block on the SM fills the tensor pipe meanwhile.
+// z-walking form of the inference convolution, for layers of NS 16-channel
+// slices.  A block keeps one (x-tile of 128 voxels, y-tile of YT rows) column
+// and walks a range of z, one input slab of each slice (a z-plane of YT + 2 rows
+// x 130 voxels in two 8-channel planes, the layout the descriptors read) at a
+// time.  An input voxel contributes to the output planes below, at and above
+// it, so the three dz taps of a (dy, dx) go into ONE MMA of N = 3 CN: its
+// accumulators are three neighbouring output planes, side by side in tensor
+// memory, and its B operand the three taps' weights in that order (dz = 1, 0,
+// -1).  A slab takes 9 x YT MMAs: with N = CN, 27 x YT were bound by their reads
+// of A from shared memory, which do not depend on N (16 -> 16 channels on
+// 100 x 512 x 512: 1.21 ms then, 0.72 ms so; 16 -> 32 on 50 x 256 x 256: 255 and
+// 173 us).
+//   An output plane adds its taps in the per-tile form's order (slice, dz, dy,
+// dx): slice s lags three planes behind slice s - 1, so that step t takes plane
+// t - 3 s of slice s and the slices work on 3 NS different output planes.  Output
+// plane o lies in slot o mod 3 NS.  Where a slab's three planes run over the end
+// of the slots, two MMAs of fewer planes take the place of one, or, with a
+// single slice, the weights are rotated (they are stored as dz = 1, 0, -1, 1, 0,
+// and a rotation is an offset into them).  No two shapes of MMA meet on an
+// accumulator without the wait at the end of a step between them.
+//   (48 -> 16 channels on 100 x 512 x 512: 3.5 ms tile by tile, 2.4 ms so; 32 -> 32
+// on 50 x 256 x 256: 405 and 364 us.)
+//   What bounds it now: an MMA of N = 48 takes some 85 cycles in all (24 of
+// arithmetic), the slab's TMA boxes of 16-byte rows (a voxel's 8 channels)
+// included; an 8-channel-plane layout of the activations would lengthen the rows.
+//   At step t thread 0 waits for the slabs, issues and commits the MMAs and, once
+// they are done, reuses the slabs' place for step t + R (one TMA box per slice
+// and half, completing on that place's mbarrier); all threads then drain the
+// output plane that the last slice completed (bias, ReLU, BF16 store, or the
+// head) and clear its accumulator.  With one slice a second block on the SM
+// fills the tensor pipe meanwhile.
 // Every wait is bounded; a wait that runs out sets *err, the block lets its
 // copies and MMAs in flight finish (bounded) and leaves.
 // ---------------------------------------------------------------------------
-template <int CN>
+template <int CN, int NS>
 struct TczShape {
-  static constexpr int YT = CN == 16 ? 4 : 2;                       // x-rows a block: 192 accumulator columns
+  static constexpr int YT = CN == 16 ? (NS == 1 ? 4 : 3) : 2;      // x-rows a block
   static constexpr int HY = YT + 2;
   static constexpr uint32_t BOX = 16u * kTcHX * HY;                 // one 8-channel plane of a slab
   static constexpr uint32_t PLANE = (BOX + 127u) / 128u * 128u;     // planes 128 bytes apart
   static constexpr uint32_t SLAB = 2u * PLANE;
-  static constexpr int R = 3;                                       // slabs in the ring
-  static constexpr uint32_t NCOLS = 256;                            // of YT x 3 x CN = 192
-  static constexpr uint32_t BHALF = 9u * 5u * CN * 16u;             // weights of one 8-channel half
+  static constexpr int R = NS == 1 ? 3 : 2;                         // steps in the ring
+  static constexpr int SLOTS = 3 * NS;                              // output planes in work
+  static constexpr uint32_t COLS = (uint32_t)YT * SLOTS * CN;
+  static constexpr uint32_t NCOLS = COLS <= 256 ? 256 : 512;
+  static constexpr int BD = NS == 1 ? 5 : 3;                        // dz blocks stored
+  static constexpr uint32_t BHALF = 9u * BD * CN * 16u;             // weights of one 8-channel half
+  static_assert(COLS <= 512, "tensor memory");
 };
 
-template <int CN>
+template <int CN, int NS>
 constexpr size_t tcz_smem() {
-  using S = TczShape<CN>;
-  return 1024 + (size_t)S::R * S::SLAB + 2 * (size_t)S::BHALF + 64;
+  using S = TczShape<CN, NS>;
+  return 1024 + (size_t)S::R * NS * S::SLAB + (size_t)NS * 2 * S::BHALF + 64;
 }
 
 __device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
@@ -531,22 +546,24 @@ __device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
       : "memory");
 }
 
-template <int CN, bool HEAD>
+template <int CN, bool HEAD, int NS>
 __global__ void __launch_bounds__(kTcThreads) k_conv3_tcz(const __grid_constant__ CUtensorMap zmap,
+                                                          const __grid_constant__ CUtensorMap skipmap, int CinA,
                                                           const __nv_bfloat16* __restrict__ Wp,
                                                           const float* __restrict__ bias,
                                                           __nv_bfloat16* __restrict__ Y, int D, int H, int W,
                                                           int zper, TcHead hd, int* __restrict__ err) {
   static_assert(CN == 16 || CN == 32, "output channels");
   static_assert(!HEAD || CN == 16, "the head takes 16 channels");
-  using S = TczShape<CN>;
-  constexpr int YT = S::YT;
+  using S = TczShape<CN, NS>;
+  constexpr int YT = S::YT, SLOTS = S::SLOTS, LAG = 3 * (NS - 1);
+  constexpr uint32_t STEP = NS * S::SLAB;
   extern __shared__ unsigned char tzraw[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tzraw) + 1023) & ~uintptr_t(1023));
-  unsigned char* slabs = base;                          // [R][2 planes] of PLANE bytes
-  unsigned char* B0 = slabs + S::R * S::SLAB;           // [2 halves][9][5][CN] x 16 B
-  uint64_t* bars = reinterpret_cast<uint64_t*>(B0 + 2 * S::BHALF);  // [0..2] slabs, [3] MMAs
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 4);
+  unsigned char* slabs = base;                          // [R][NS][2 planes] of PLANE bytes
+  unsigned char* B0 = slabs + S::R * STEP;              // [NS][2 halves][9][BD][CN] x 16 B
+  uint64_t* bars = reinterpret_cast<uint64_t*>(B0 + NS * 2 * S::BHALF);  // [0..R-1] slabs, [R] MMAs
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + S::R + 1);
   int* s_ok = reinterpret_cast<int*>(tslot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nbx = W / kTcX, nby = (H + YT - 1) / YT;
@@ -561,15 +578,17 @@ __global__ void __launch_bounds__(kTcThreads) k_conv3_tcz(const __grid_constant_
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (tid == 0) {
-    for (int i = 0; i < 4; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(saddr(bars + i)) : "memory");
+    for (int i = 0; i <= S::R; ++i)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(saddr(bars + i)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     *s_ok = 1;
   }
-  // weights: row (half, dy dx, j, co) is tap dz = 1, 0, -1, 1, 0 for j = 0..4 of the layer's [half][27][CN] rows
-  for (int e = tid; e < 2 * 9 * 5 * CN; e += kTcThreads) {
-    const int co = e % CN, j = e / CN % 5, t9 = e / (5 * CN) % 9, half = e / (45 * CN);
+  // weights: row (slice, half, dy dx, j, co) is tap dz = 1, 0, -1, 1, 0 for j = 0..4 of the layer's
+  // [slice][half][27][CN] rows
+  for (int e = tid; e < NS * 2 * 9 * S::BD * CN; e += kTcThreads) {
+    const int co = e % CN, j = e / CN % S::BD, t9 = e / (S::BD * CN) % 9, sh = e / (9 * S::BD * CN);
     const int kz = (2 * j + 2) % 3;  // 2, 1, 0, 2, 1
-    reinterpret_cast<uint4*>(B0)[e] = __ldg(reinterpret_cast<const uint4*>(Wp) + (half * 27 + kz * 9 + t9) * CN + co);
+    reinterpret_cast<uint4*>(B0)[e] = __ldg(reinterpret_cast<const uint4*>(Wp) + (sh * 27 + kz * 9 + t9) * CN + co);
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes -> tensor-core reads
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -577,74 +596,109 @@ __global__ void __launch_bounds__(kTcThreads) k_conv3_tcz(const __grid_constant_
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tbase = *tslot;
   const uint32_t twarp = tbase + ((uint32_t)(warp * 32) << 16);  // this warp's lanes
-  const uint32_t idesc = instr_desc(3 * CN);
-  const uint32_t s0 = saddr(slabs), b0 = saddr(B0);
-  uint32_t phase[S::R] = {0u, 0u, 0u};  // thread 0: parity of each slot's next completion
-  bool busy[S::R] = {false, false, false};  // a copy into the slot not yet awaited
-  uint32_t pm = 0;                      // parity of the MMA barrier
+  const uint32_t s0 = saddr(slabs), b0 = saddr(B0), bar_mma = saddr(bars + S::R);
+  uint32_t phase = 0;      // thread 0: parity of each place's next completion, a bit each
+  uint32_t busy = 0;       // copies into a place not yet awaited, a bit each
+  uint32_t pm = 0;         // parity of the MMA barrier
   bool mma_busy = false;
   bool ok = true;
-  auto load_slab = [&](int z, uint32_t sl) {  // thread 0
-    const uint32_t bar = saddr(bars + sl);
-    busy[sl] = true;
-    mbar_expect_tx(bar, 2u * S::BOX);
+  // slice s's plane at step t is t - 3 s; it has one while that is in [zb - 1, ze]
+  const int tb = zb - 1, te = ze + LAG;
+  auto load_step = [&](int t, uint32_t pl) {  // thread 0
+    const uint32_t bar = saddr(bars + pl);
+    int n = 0;
 #pragma unroll
-    for (int p = 0; p < 2; ++p)
-      tma_load_4d(s0 + sl * S::SLAB + (uint32_t)p * S::PLANE, &zmap, 8 * p, x0 - 1, y0 - 1, z, bar);
+    for (int s = 0; s < NS; ++s) n += t - 3 * s >= tb && t - 3 * s <= ze;
+    busy |= 1u << pl;
+    mbar_expect_tx(bar, (uint32_t)n * 2u * S::BOX);
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      const int z = t - 3 * s;  // planes outside the volume read as zeros
+      if (z < tb || z > ze) continue;
+      const bool skip = 16 * s >= CinA;
+      const CUtensorMap* const map = skip ? &skipmap : &zmap;
+      const int ch = 16 * s - (skip ? CinA : 0);
+#pragma unroll
+      for (int p = 0; p < 2; ++p)
+        tma_load_4d(s0 + pl * STEP + (uint32_t)s * S::SLAB + (uint32_t)p * S::PLANE, map, ch + 8 * p, x0 - 1, y0 - 1, z,
+                    bar);
+    }
   };
-  // the ring starts with plane zb - 1 in slot 0; planes outside the volume read as zeros
-  if (tid == 0 && zb < ze)
-    for (int i = 0; i < S::R && zb - 1 + i <= ze; ++i) load_slab(zb - 1 + i, (uint32_t)i);
+  // the 9 x YT MMAs of a slab: A descriptor of the slab, B of the first tap's weights, slot, number of planes
+  auto issue = [&](uint64_t ad, uint64_t bd, int slot, uint32_t idesc) {
 #pragma unroll
-  for (int i = 0; i < YT * 3 * CN / 16; ++i) tmem_zero16(twarp + (uint32_t)(16 * i));
+    for (int k = 0; k < 9; ++k)
+#pragma unroll
+      for (int m = 0; m < YT; ++m)
+        mma_bf16_ss(tbase + (uint32_t)((m * SLOTS + slot) * CN), ad + (uint64_t)((m + k / 3) * kTcHX + k % 3),
+                    bd + (uint64_t)(k * S::BD * CN), idesc, 1u);
+  };
+  if (tid == 0 && zb < ze)
+    for (int i = 0; i < S::R && tb + i <= te; ++i) load_step(tb + i, (uint32_t)i);
+#pragma unroll
+  for (uint32_t i = 0; i < S::COLS / 16; ++i) tmem_zero16(twarp + 16 * i);
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  uint32_t r3 = 0;  // (z - zb + 1) mod 3: slab z's slot in the ring and output plane z's accumulator
-  for (int z = zb - 1; z <= ze; ++z) {
-    const uint32_t below = r3 == 0 ? 2u : r3 - 1u;  // output plane z - 1's accumulator
+  uint32_t pl = 0;          // (t - tb) mod R: the step's place in the ring
+  int first = SLOTS - 1;    // (t - zb) mod SLOTS: the slot of slice 0's lowest output plane, t - 1
+  for (int t = tb; t <= te; ++t) {
+    // the last slice's lowest plane, complete after this step
+    int done = first - LAG % SLOTS;
+    if (done < 0) done += SLOTS;
     if (tid == 0) {
       if (ok) {
-        ok = mbar_wait(saddr(bars + r3), phase[r3]);
+        ok = mbar_wait(saddr(bars + pl), phase >> pl & 1u);
         if (ok) {
-          phase[r3] ^= 1u;
-          busy[r3] = false;
+          phase ^= 1u << pl;
+          busy &= ~(1u << pl);
         }
       }
       if (ok) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint64_t ad = smem_desc(s0 + r3 * S::SLAB, S::PLANE, 128);
-        // slots hold planes with dz (1, 0, -1) from slot `below` on
-        const uint64_t bd = smem_desc(b0, S::BHALF, 128) + (uint64_t)((3u - below) % 3u * CN);
-#pragma unroll
-        for (int k = 0; k < 9; ++k)
-#pragma unroll
-          for (int m = 0; m < YT; ++m)
-            mma_bf16_ss(tbase + (uint32_t)(m * 3 * CN), ad + (uint64_t)((m + k / 3) * kTcHX + k % 3),
-                        bd + (uint64_t)(k * 5 * CN), idesc, 1u);
-        mma_commit(saddr(bars + 3));
+#pragma unroll 1
+        for (int s = 0; s < NS; ++s) {
+          if (t - 3 * s < tb || t - 3 * s > ze) continue;
+          const uint64_t ad = smem_desc(s0 + pl * STEP + (uint32_t)s * S::SLAB, S::PLANE, 128);
+          const uint64_t bd = smem_desc(b0 + (uint32_t)(s * 2) * S::BHALF, S::BHALF, 128);
+          if constexpr (NS == 1) {
+            issue(ad, bd + (uint64_t)((3 - first) % 3 * CN), 0, instr_desc(3 * CN));
+          } else {
+            int slot = first - 3 * s;
+            if (slot < 0) slot += SLOTS;
+            const int n = SLOTS - slot;  // planes before the end of the slots
+            if (n >= 3) {
+              issue(ad, bd, slot, instr_desc(3 * CN));
+            } else {
+              issue(ad, bd, slot, n == 2 ? instr_desc(2 * CN) : instr_desc(CN));
+              issue(ad, bd + (uint64_t)(n * CN), 0, n == 2 ? instr_desc(CN) : instr_desc(2 * CN));
+            }
+          }
+        }
+        mma_commit(bar_mma);
         mma_busy = true;
-        ok = mbar_wait(saddr(bars + 3), pm);
+        ok = mbar_wait(bar_mma, pm);
         if (ok) {
           pm ^= 1u;
           mma_busy = false;
         }
-        if (ok && z + S::R <= ze) load_slab(z + S::R, r3);
+        if (ok && t + S::R <= te) load_step(t + S::R, pl);
       }
       if (!ok) *s_ok = 0;
     }
     __syncthreads();
     if (!*s_ok) break;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const int zo = t - LAG - 1;  // the plane in slot `done`
     const int xx = x0 + warp * 32 + lane;
 #pragma unroll 1
     for (int m = 0; m < YT; ++m) {
-      const uint32_t acc = twarp + (uint32_t)(m * 3 * CN) + below * CN;
+      const uint32_t acc = twarp + (uint32_t)((m * SLOTS + done) * CN);
       const int yy = y0 + m;
-      const long long vox = ((long long)(z - 1) * H + yy) * W + xx;
+      const long long vox = ((long long)zo * H + yy) * W + xx;
       float zsum = 0.f;
       if constexpr (HEAD) zsum = hd.w[16];
-      if (z > zb) {
+      if (zo >= zb) {
 #pragma unroll
         for (int c16 = 0; c16 < CN / 16; ++c16) {
           float v[16];
@@ -681,19 +735,20 @@ __global__ void __launch_bounds__(kTcThreads) k_conv3_tcz(const __grid_constant_
 #pragma unroll
       for (int c16 = 0; c16 < CN / 16; ++c16) tmem_zero16(acc + (uint32_t)(c16 * 16));
     }
-    // every thread's accumulator reads and clears come before the next slab's MMAs
+    // every thread's accumulator reads and clears come before the next step's MMAs
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    r3 = r3 == 2 ? 0u : r3 + 1u;
+    pl = pl + 1 == S::R ? 0u : pl + 1;
+    first = first + 1 == SLOTS ? 0 : first + 1;
   }
   if (tid == 0 && !ok) {
     atomicExch(err, 1);
     // a last bounded wait for the copies and MMAs still in flight before the
     // shared and tensor memory are released
-    if (mma_busy) mbar_wait(saddr(bars + 3), pm);
+    if (mma_busy) mbar_wait(bar_mma, pm);
     for (int i = 0; i < S::R; ++i)
-      if (busy[i]) mbar_wait(saddr(bars + i), phase[i]);
+      if (busy >> i & 1u) mbar_wait(saddr(bars + i), phase >> i & 1u);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -720,8 +775,9 @@ EncodeTiledFn encode_tiled() {
 }
 
 template <int CN, bool HEAD>
-cudaError_t tcb_launch(const TcMap& m, const TcMap& ms, int CinA, int Cin, const __nv_bfloat16* Wp, const float* bias, __nv_bfloat16* Y, int D,
-                       int H, int W, const TcHead& hd, int* err, cudaStream_t st) {
+cudaError_t tcb_launch(const TcMap& m, const TcMap& ms, int CinA, int Cin, const __nv_bfloat16* Wp,
+                       const float* bias, __nv_bfloat16* Y, int D, int H, int W, const TcHead& hd, int* err,
+                       cudaStream_t st) {
   constexpr size_t smem = tcb_smem<CN>();
   static bool opted = false;
   if (!opted) {
@@ -770,7 +826,11 @@ bool tc_map_encode(TcMap* m, const __nv_bfloat16* X, int C, int D, int H, int W)
 }
 
 // x-rows a block of the z-walking form takes
-int tcz_rows(int Cout) { return Cout == 16 ? TczShape<16>::YT : TczShape<32>::YT; }
+int tcz_rows(int Cin, int Cout) {
+  if (Cin == 48) return TczShape<16, 3>::YT;
+  if (Cin == 32) return TczShape<32, 2>::YT;
+  return Cout == 16 ? TczShape<16, 1>::YT : TczShape<32, 1>::YT;
+}
 
 bool tc_zmap_encode(TcMap* m, const __nv_bfloat16* X, int C, int D, int H, int W, int rows) {
   const EncodeTiledFn enc = encode_tiled();
@@ -789,23 +849,21 @@ bool tc_zmap_encode(TcMap* m, const __nv_bfloat16* X, int C, int D, int H, int W
   return true;
 }
 
-// 16 input channels only: 48 channels would add their three slices plane by plane
-// instead of one after another (other roundings), and walking z in the old order
-// the ring and the
-// weights fill the shared memory of one block an SM, and that layer measured
-// slower walking z (a block's loads, MMAs and epilogue then have nothing to
-// overlap with) than in the per-tile kernel.
+// The layers whose output planes in work (3 for each 16-channel slice, at least
+// two rows of them) fit tensor memory.
 bool tcz_supported(int W, int Cin, int Cout) {
-  return W % kTcX == 0 && Cin == 16 && (Cout == 16 || Cout == 32) && encode_tiled() != nullptr;
+  const bool fits = (Cin == 16 && (Cout == 16 || Cout == 32)) || (Cin == 32 && Cout == 32) || (Cin == 48 && Cout == 16);
+  return W % kTcX == 0 && fits && encode_tiled() != nullptr;
 }
 
 namespace {
-template <int CN, bool HEAD>
-cudaError_t tcz_launch(const TcMap& m, const __nv_bfloat16* Wp, const float* bias, __nv_bfloat16* Y, int D, int H,
-                       int W, const TcHead& hd, int* err, cudaStream_t st) {
-  constexpr int YT = TczShape<CN>::YT;
-  constexpr size_t smem = tcz_smem<CN>();
-  const auto kern = k_conv3_tcz<CN, HEAD>;
+template <int CN, bool HEAD, int NS>
+cudaError_t tcz_launch(const TcMap& m, const TcMap& skip, int CinA, const __nv_bfloat16* Wp, const float* bias,
+                       __nv_bfloat16* Y, int D, int H, int W, const TcHead& hd, int* err, cudaStream_t st) {
+  using S = TczShape<CN, NS>;
+  constexpr int YT = S::YT;
+  constexpr size_t smem = tcz_smem<CN, NS>();
+  const auto kern = k_conv3_tcz<CN, HEAD, NS>;
   static bool opted = false;
   if (!opted) {
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -817,21 +875,21 @@ cudaError_t tcz_launch(const TcMap& m, const __nv_bfloat16* Wp, const float* bia
     cudaGetLastError();
     per_sm = 1;
   }
-  per_sm = std::min(per_sm, (int)(512 / TczShape<CN>::NCOLS));  // tensor memory
+  per_sm = std::min(per_sm, (int)(512 / S::NCOLS));  // tensor memory
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) !=
                                                  cudaSuccess) {
     cudaGetLastError();
     sms = 148;
   }
-  // z-ranges per (x, y) column: whole waves of blocks against the two slabs each range reads beyond its own
+  // z-ranges per (x, y) column: whole waves of blocks against the steps each range takes beyond its planes
   const long long xy = (long long)(W / kTcX) * ((H + YT - 1) / YT);
   int zper = D;
   double best = 1e300;
   for (int n = 1; n <= D && n <= 64; ++n) {
     const int len = (D + n - 1) / n;
     const double waves = std::ceil((double)xy * ((D + len - 1) / len) / ((double)sms * per_sm));
-    const double cost = waves * (len + 3);
+    const double cost = waves * (len + 3 * NS);
     if (cost < best * 0.999) {
       best = cost;
       zper = len;
@@ -839,20 +897,25 @@ cudaError_t tcz_launch(const TcMap& m, const __nv_bfloat16* Wp, const float* bia
   }
   const long long blocks = xy * ((D + zper - 1) / zper);
   if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-  CUtensorMap map;
+  CUtensorMap map, smap;
   std::memcpy(&map, m.bytes, sizeof(map));
-  kern<<<(unsigned)blocks, kTcThreads, smem, st>>>(map, Wp, bias, Y, D, H, W, zper, hd, err);
+  std::memcpy(&smap, skip.bytes, sizeof(smap));
+  kern<<<(unsigned)blocks, kTcThreads, smem, st>>>(map, smap, CinA, Wp, bias, Y, D, H, W, zper, hd, err);
   return cudaGetLastError();
 }
 }  // namespace
 
-cudaError_t conv3_tcz(const TcMap& zmap, int Cin, const __nv_bfloat16* Wp, const float* bias, int Cout,
-                      __nv_bfloat16* Y, int D, int H, int W, const TcHead* head, int* err, cudaStream_t st) {
-  if (!tcz_supported(W, Cin, Cout) || (head && Cout != 16)) return cudaErrorInvalidValue;
+cudaError_t conv3_tcz(const TcMap& zmap, const TcMap& skipmap, int CinA, int Cin, const __nv_bfloat16* Wp,
+                      const float* bias, int Cout, __nv_bfloat16* Y, int D, int H, int W, const TcHead* head, int* err,
+                      cudaStream_t st) {
+  if (!tcz_supported(W, Cin, Cout) || CinA % 16 != 0 || CinA > Cin || (head && (Cin != 16 || Cout != 16)))
+    return cudaErrorInvalidValue;
   const TcHead hd = head ? *head : TcHead{};
-  if (head) return tcz_launch<16, true>(zmap, Wp, bias, Y, D, H, W, hd, err, st);
-  return Cout == 16 ? tcz_launch<16, false>(zmap, Wp, bias, Y, D, H, W, hd, err, st)
-                    : tcz_launch<32, false>(zmap, Wp, bias, Y, D, H, W, hd, err, st);
+  if (head) return tcz_launch<16, true, 1>(zmap, skipmap, CinA, Wp, bias, Y, D, H, W, hd, err, st);
+  if (Cin == 48) return tcz_launch<16, false, 3>(zmap, skipmap, CinA, Wp, bias, Y, D, H, W, hd, err, st);
+  if (Cin == 32) return tcz_launch<32, false, 2>(zmap, skipmap, CinA, Wp, bias, Y, D, H, W, hd, err, st);
+  return Cout == 16 ? tcz_launch<16, false, 1>(zmap, skipmap, CinA, Wp, bias, Y, D, H, W, hd, err, st)
+                    : tcz_launch<32, false, 1>(zmap, skipmap, CinA, Wp, bias, Y, D, H, W, hd, err, st);
 }
 
 bool conv3_tc_bf16_supported(int D, int H, int W, int Cin, int Cout) {
@@ -870,7 +933,8 @@ cudaError_t tc_weights(const float* w, int Cout, int Cin, __nv_bfloat16* wp, cud
 }
 
 cudaError_t conv3_tc_bf16(const TcMap& xmap, const TcMap& skipmap, int CinA, int Cin, const __nv_bfloat16* Wp,
-                          const float* bias, int Cout, __nv_bfloat16* Y, int D, int H, int W, const TcHead* head, int* err, cudaStream_t st) {
+                          const float* bias, int Cout, __nv_bfloat16* Y, int D, int H, int W, const TcHead* head,
+                          int* err, cudaStream_t st) {
   if (!conv3_tc_bf16_supported(D, H, W, Cin, Cout) || CinA % 16 != 0 || CinA > Cin) return cudaErrorInvalidValue;
   const TcHead hd = head ? *head : TcHead{};
   if (head) {

@@ -37,18 +37,20 @@ size_t tc_weights_elems(int Cout, int Cin);
 cudaError_t tc_weights(const float* w, int Cout, int Cin, __nv_bfloat16* wp, cudaStream_t st);
 // The first CinA of the Cin input channels are xmap's, the others skipmap's
 // (a second tensor of the same volume; CinA = Cin: none).
-cudaError_t conv3_tc_bf16(const TcMap& xmap, const TcMap& skipmap, int CinA, int Cin, const __nv_bfloat16* Wp, const float* bias, int Cout,
-                          __nv_bfloat16* Y, int D, int H, int W, const TcHead* head, int* err, cudaStream_t st);
+cudaError_t conv3_tc_bf16(const TcMap& xmap, const TcMap& skipmap, int CinA, int Cin, const __nv_bfloat16* Wp,
+                          const float* bias, int Cout, __nv_bfloat16* Y, int D, int H, int W, const TcHead* head,
+                          int* err, cudaStream_t st);
 
-// The z-walking form of the same convolution (16 input channels, 16 or 32
-// output channels; the head with 16): a block walks z over one (x, y) tile
-// with a ring of three input planes, each loaded once, through a tensor map
-// made by tc_zmap_encode with `rows` = tcz_rows(Cout) + 2.
+// The z-walking form of the same convolution (16 -> 16 and 32 channels, 32 -> 32,
+// 48 -> 16; the head after 16 -> 16): a block walks z over one (x, y) tile, each
+// input plane loaded once through tensor maps made by tc_zmap_encode with
+// `rows` = tcz_rows(Cin, Cout) + 2.
 bool tcz_supported(int W, int Cin, int Cout);
-int tcz_rows(int Cout);
+int tcz_rows(int Cin, int Cout);
 bool tc_zmap_encode(TcMap* m, const __nv_bfloat16* X, int C, int D, int H, int W, int rows);
-cudaError_t conv3_tcz(const TcMap& zmap, int Cin, const __nv_bfloat16* Wp, const float* bias, int Cout,
-                      __nv_bfloat16* Y, int D, int H, int W, const TcHead* head, int* err, cudaStream_t st);
+cudaError_t conv3_tcz(const TcMap& zmap, const TcMap& skipmap, int CinA, int Cin, const __nv_bfloat16* Wp,
+                      const float* bias, int Cout, __nv_bfloat16* Y, int D, int H, int W, const TcHead* head, int* err,
+                      cudaStream_t st);
 
 // dW[co][tap][ci] += sum over voxels of dY[v][co] X[v + off][ci], FP32
 // channels-last operands rounded to BF16 (rihvr_unet_grad.cu); Cin a multiple
