@@ -143,8 +143,9 @@ int rihvr_plane_list(const rihvr_params* params, double* z_out);
 /* SparseCompressiveHolo::SparseCompressiveHolo(Hologram)
  * (src/core/sparse_compressive_holo.cu:58-135).  width x height is the padded
  * hologram size.  Each side is even, 16..4096, with prime factors 2, 3, 5 and 7
- * only (the reference needs multiples of 16); square planes of side 32, 48, 64,
- * 128, 256, 384, 512, 640, 768, 1024 or 2304 take the fastest FFT passes. */
+ * only (the reference needs multiples of 16); sides of 32, 48, 64, 128, 256, 384,
+ * 512, 640, 768, 1024 and 2304 take the fastest FFT passes (row passes by the
+ * width, column passes by the height). */
 int rihvr_create(const rihvr_params* params, int width, int height, rihvr_ctx** out);
 
 /* SparseCompressiveHolo::destroy (:137-146). */
@@ -266,14 +267,14 @@ int rihvr_autotune(rihvr_ctx* ctx, double* best_ms);
  * 2 streaming in 2-warp blocks, 3 streaming in 4-warp blocks, 4 streaming in
  * one launch where 6-10 TV iterations would take two); 0 means the built-in
  * choice.  adj_recurrence receives the
- * adjoint column pass's variant for evenly spaced planes (square planes of side
- * 32 to 2304 except 640): 0 transfer function evaluated at every
+ * adjoint column pass's variant for evenly spaced planes (heights of the fastest
+ * passes except 640): 0 transfer function evaluated at every
  * plane, 1 advanced by a recurrence with the inter-stage twiddles regenerated
  * each plane, 2 the recurrence with the twiddles kept in registers (these two
  * up to side 1024, except 384 and 768), 3 the recurrence with the twiddles
  * read from a per-block shared table.  fwd_horner receives the forward column
  * pass's variant: 1 when it sums over evenly spaced planes by Horner's scheme
- * (square planes of side 32 to 512 and 1024) with its input strip
+ * (heights of 32 to 512 and 1024) with its input strip
  * double-buffered, 2 for the same sum with the strip staged in the exchange
  * buffer and a shared twiddle table (also sides 384, 768 and 2304), 3 for
  * that form with the strip loaded by TMA, else 0.  Any pointer may be NULL. */
@@ -345,7 +346,10 @@ int rihvr_slab_iterate(rihvr_ctx* const* ctxs, int n, int iterations, const rihv
  * RIHVR_ERR_INVALID_FILE, context unchanged);
  * further rihvr_iterate calls then continue the solve bit for bit as if it
  * had not stopped (with the same launch shapes: both contexts untuned, or
- * tuned alike).  The file takes about 2 x Nz x H x W x storage size bytes. */
+ * tuned alike).  The file takes about 2 x Nz x H x W x storage size bytes.
+ * Files of version 2, which lack the spectrum of the last estimate that version
+ * 3 appends, load too; that spectrum is then computed, so the continued solve
+ * agrees up to its FP32 rounding. */
 int rihvr_save_state(rihvr_ctx* ctx, const char* path);
 int rihvr_load_state(rihvr_ctx* ctx, const char* path);
 

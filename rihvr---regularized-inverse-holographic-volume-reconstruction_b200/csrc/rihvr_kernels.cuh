@@ -55,7 +55,7 @@ struct ProxArgs {
 };
 
 bool line_size_supported(int n);
-// sides the generic line FFT handles (prime factors 2, 3, 5, 7; up to 8192)
+// sides the line FFTs without a register-resident split handle (prime factors 2, 3, 5, 7)
 bool generic_size_supported(int n);
 // message returned by rihvr_last_error on this thread
 void set_last_error(const char* msg);
@@ -74,12 +74,12 @@ int segment_volume(int storage, const void* P, const void* Pprev, float beta, in
                    rihvr_segment_info* info, SegWorkspace* ws, cudaStream_t st);
 size_t max_partial_blocks(int W, int H, int Nz);
 
-// square sizes whose adjoint column pass has the recurrence variant
+// planes whose adjoint column pass has the recurrence variant
 bool adj_recurrence_supported(int W, int H, int rec_mode = 2);
 // the variant (rec_mode) the adjoint column pass takes untuned for evenly spaced planes
 int adj_col_builtin(int W, int H, int Nz);
 // dz_uniform != 0: the planes are evenly spaced by dz_uniform (z_{k+1} - z_k,
-// exact in FP64), which lets the square fast sizes advance the transfer
+// exact in FP64), which lets the fast heights advance the transfer
 // function by a recurrence (rec_mode 1: twiddles regenerated each plane, three
 // blocks an SM; 2: twiddles kept in registers, two blocks an SM; 3: twiddles
 // from a per-block shared table, three blocks an SM); rec_mode 0 or
@@ -89,7 +89,7 @@ cudaError_t launch_adj_col(const float2* Rs, const double* cturn, const double* 
                            int rec_mode = 0);
 cudaError_t launch_rows(int inverse, int in_kind, const void* in, int out_kind, void* out, int W,
                         long long nlines, float scale, cudaStream_t st);
-// dz_uniform != 0 (evenly spaced planes): square staged sizes sum over z by
+// dz_uniform != 0 (evenly spaced planes): staged heights sum over z by
 // Horner's scheme with the rotation H'_dz (fwd_horner_supported); horner_mode
 // 1 stages T in its own double buffer (two blocks an SM), 2 in the exchange
 // buffer with the twiddles in a shared table (three blocks an SM), 3 the same

@@ -1381,10 +1381,10 @@ bool usable_in_place(const rihvr_ctx* c, const void* p) {
 int validate(const rihvr_params* p, int W, int H) {
   if (!p) return fail(RIHVR_ERR_INVALID_ARGUMENT, "params is NULL");
   if (W <= 0 || H <= 0) return fail(RIHVR_ERR_INVALID_ARGUMENT, "width and height must be positive");
-  // Square planes of side 32, 48, 64, 128, 256, 384, 512, 640, 768, 1024 or 2304 take the
-  // register-resident FFT passes; any other even width and height from 16 to
-  // 4096 whose prime factors are 2, 3, 5 and 7 takes the generic passes (the
-  // reference needs multiples of 16, :126, 1948).
+  // Sides of 32, 48, 64, 128, 256, 384, 512, 640, 768, 1024 and 2304 take the
+  // register-resident FFT passes (rows by the width, columns by the height); any
+  // other even side from 16 to 4096 whose prime factors are 2, 3, 5 and 7 takes
+  // the staged line FFTs (the reference needs multiples of 16, :126, 1948).
   for (int n : {W, H}) {
     if (n < 16 || (n & 1) || !(line_size_supported(n) || generic_size_supported(n)))
       return fail(RIHVR_ERR_UNSUPPORTED_SIZE,
