@@ -682,9 +682,15 @@ int segment_impl(SRC src, int W, int H, int Nz, const rihvr_segment_params* sp, 
   const size_t o_q = kStoreQ ? c0.add<float>((size_t)nvox) : 0;
   // room for the later steps when few voxels are on, as particles have it (one
   // in 200; about 52 bytes each), so that a call allocates once
-  const size_t spare = 65536 + (size_t)nvox / 4;
-  const size_t o_spare = c0.add<unsigned char>(spare);
-  SCK(ws.reserve(0, c0.bytes));
+  size_t spare = 65536 + (size_t)nvox / 4;
+  const size_t without = c0.bytes, o_spare = c0.add<unsigned char>(spare);
+  cudaError_t e0 = ws.reserve(0, c0.bytes);
+  if (e0 == cudaErrorMemoryAllocation) {  // the steps then allocate their own
+    cudaGetLastError();
+    spare = 0;
+    e0 = ws.reserve(0, without);
+  }
+  SCK(e0);
   unsigned char* const m0 = ws.p[0];
   unsigned* const maxbits = reinterpret_cast<unsigned*>(m0 + o_max);
   int* const err = reinterpret_cast<int*>(m0 + o_err);
