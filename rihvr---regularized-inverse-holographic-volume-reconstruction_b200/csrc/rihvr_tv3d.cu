@@ -11,7 +11,7 @@
 // stencil to X1 give the estimate, with one volume in and one out instead of
 // four in and three out for each step (the dual form moved 96 bytes a voxel
 // and step, a stencil pass 16).  At 256 x 256 x 100 with 5 steps the prox took
-// 817 us in the dual form and 239 us here.
+// 817 us in the dual form and 207 us here.
 #include <algorithm>
 #include <cmath>
 #include <utility>
@@ -242,23 +242,40 @@ cudaError_t launch_tv3(const ProxArgs& a, float2* X1, float2* other, const float
 // columns walks a run of planes, so that the plane before it (which the 3-D TV
 // norms need) is at hand; left neighbours move by shuffles, upper ones come
 // from the caches.
+//
+// What bounds it: latency.  A plane's loads are issued while the plane before
+// is worked on, as stored (a conversion would wait for them); with the loads of
+// each plane after the last one's sums, 256 x 256 x 100 took 96 us with the norm
+// terms, 67 us so (40 us at the memory's rate).
 // ---------------------------------------------------------------------------
-template <typename ST>
-__device__ __forceinline__ void x_pair(const ST* P, const ST* Pp, float beta, size_t i, float2 (&x)[2],
-                                       float2 (&p)[2]) {
-  float2 q[2];
-  Pair<ST>::ld(P + i, p[0], p[1]);
-  Pair<ST>::ld(Pp + i, q[0], q[1]);
-#pragma unroll
-  for (int c = 0; c < 2; ++c)
-    x[c] = make_float2(fmaf(beta, p[c].x - q[c].x, p[c].x), fmaf(beta, p[c].y - q[c].y, p[c].y));
+__device__ __forceinline__ float2 momentum(float2 p, float2 q, float beta) {
+  return make_float2(fmaf(beta, p.x - q.x, p.x), fmaf(beta, p.y - q.y, p.y));
 }
 
-__device__ __forceinline__ void y_pair(const float2* Y, size_t i, float T, int faithful, float2 (&v)[2]) {
-  Pair<float2>::ld(Y + i, v[0], v[1]);
-  v[0] = shrink(v[0], T, faithful);
-  v[1] = shrink(v[1], T, faithful);
-}
+// two voxels of Y, P and Pprev as stored
+template <typename ST>
+struct Raw6 {
+  float4 y;
+  typename Raw2<ST>::T p, q;
+  __device__ __forceinline__ void ld(const float2* Y, const ST* P, const ST* Pp, size_t i) {
+    y = Raw2<float2>::ld(Y + i);
+    p = Raw2<ST>::ld(P + i);
+    q = Raw2<ST>::ld(Pp + i);
+  }
+  // the thresholded estimate v, the momentum point x and P itself
+  __device__ __forceinline__ void get(float T, float beta, int faithful, float2 (&v)[2], float2 (&x)[2],
+                                      float2 (&pv)[2]) const {
+    float2 qv[2];
+    Raw2<float2>::cvt(y, v[0], v[1]);
+    Raw2<ST>::cvt(p, pv[0], pv[1]);
+    Raw2<ST>::cvt(q, qv[0], qv[1]);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      v[c] = shrink(v[c], T, faithful);
+      x[c] = momentum(pv[c], qv[c], beta);
+    }
+  }
+};
 
 template <typename ST, bool NORMS>
 __global__ void __launch_bounds__(FLAT_THREADS) k_prox6_finish(ProxArgs a0, const float2* __restrict__ Y,
@@ -276,7 +293,7 @@ __global__ void __launch_bounds__(FLAT_THREADS) k_prox6_finish(ProxArgs a0, cons
   const bool ok = xx < W && yy < H;
   const size_t e = ok ? (size_t)yy * W + xx : 0;
   // the column left of the block's and the row above
-  const size_t el = ok ? (size_t)yy * W + (xx > 0 ? xx - 2 : W - 2) : 0;
+  const size_t el = ok ? (size_t)yy * W + (xx > 0 ? xx - 1 : W - 1) : 0;
   const size_t eu = ok ? (size_t)(yy > 0 ? yy - 1 : H - 1) * W + xx : 0;
   float wr, wi;
   restart_w(e, a.faithful, &wr, &wi);  // e is even: both columns are in the same 512
@@ -285,20 +302,50 @@ __global__ void __launch_bounds__(FLAT_THREADS) k_prox6_finish(ProxArgs a0, cons
   for (int k = 0; k < kNumSums; ++k) acc[k] = 0.0;
   float2 pb[2], xb[2];  // p and x on the plane before
   if (NORMS) {
-    const size_t zb = (size_t)(z0 > 0 ? z0 - 1 : Nz - 1) * HW;
+    Raw6<ST> r;
     float2 t[2];
-    y_pair(Y, zb + e, T, a.faithful, pb);
-    x_pair(P, Pp, a.beta, zb + e, xb, t);
+    r.ld(Y, P, Pp, (size_t)(z0 > 0 ? z0 - 1 : Nz - 1) * HW + e);
+    r.get(T, a.beta, a.faithful, pb, xb, t);
   }
+  // the plane to come, as stored: this pair, the one above and lane 0's left neighbour
+  Raw6<ST> rc, ru;
+  float4 rg;
+  float2 ly;
+  ST lp, lq;
+  auto request = [&](int z) {
+    const size_t zo = (size_t)z * HW;
+    rc.ld(Y, P, Pp, zo + e);
+    rg = Raw2<float2>::ld(a.G + zo + e);
+    if (NORMS) {
+      ru.ld(Y, P, Pp, zo + eu);
+      if (lane == 0) {
+        ly = Y[zo + el];
+        lp = P[zo + el];
+        lq = Pp[zo + el];
+      }
+    }
+  };
+  if (z0 < z1) request(z0);
 #pragma unroll 1
   for (int z = z0; z < z1; ++z) {
-    const size_t zo = (size_t)z * HW;
-    float2 p[2], x[2], y0[2], g[2];
-    y_pair(Y, zo + e, T, a.faithful, p);
-    x_pair(P, Pp, a.beta, zo + e, x, y0);
-    Pair<float2>::ld(a.G + zo + e, g[0], g[1]);
+    float2 p[2], x[2], y0[2], g[2], pu[2], xu[2], pl[2], xl[2];
+    rc.get(T, a.beta, a.faithful, p, x, y0);
+    Raw2<float2>::cvt(rg, g[0], g[1]);
+    if (NORMS) {
+      float2 t[2];
+      ru.get(T, a.beta, a.faithful, pu, xu, t);
+      pl[1] = p[0];
+      xl[1] = x[0];
+      pl[0] = shfl_up2(p[1]);
+      xl[0] = shfl_up2(x[1]);
+      if (lane == 0) {
+        pl[0] = shrink(ly, T, a.faithful);
+        xl[0] = momentum(Store<ST>::ld(&lp), Store<ST>::ld(&lq), a.beta);
+      }
+    }
+    if (z + 1 < z1) request(z + 1);
     if (ok) {
-      Raw2<ST>::st(Pn + zo + e, p[0], p[1]);
+      Raw2<ST>::st(Pn + (size_t)z * HW + e, p[0], p[1]);
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         const float2 d = csub(p[c], x[c]);
@@ -306,26 +353,7 @@ __global__ void __launch_bounds__(FLAT_THREADS) k_prox6_finish(ProxArgs a0, cons
         acc[SUM_LIM2] += (double)cabs2(d);
         const float2 u = csub(x[c], p[c]), v = csub(p[c], y0[c]);
         acc[SUM_RS] += (double)(wr * u.x * v.x) + (double)(wi * u.y * v.y);
-      }
-    }
-    if (NORMS) {
-      float2 pl[2], xl[2], pu[2], xu[2], t[2];
-      pl[1] = p[0];
-      xl[1] = x[0];
-      pl[0] = shfl_up2(p[1]);
-      xl[0] = shfl_up2(x[1]);
-      if (lane == 0) {
-        y_pair(Y, zo + el, T, a.faithful, t);
-        pl[0] = t[1];
-        float2 u[2];
-        x_pair(P, Pp, a.beta, zo + el, t, u);
-        xl[0] = t[1];
-      }
-      y_pair(Y, zo + eu, T, a.faithful, pu);
-      x_pair(P, Pp, a.beta, zo + eu, xu, t);
-      if (ok) {
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
+        if (NORMS) {
           acc[SUM_L1P] += (double)norm_sqrt(cabs2(p[c]));
           acc[SUM_TVP] += (double)norm_sqrt(cabs2(csub(pl[c], p[c])) + cabs2(csub(pu[c], p[c])) +
                                             cabs2(csub(pb[c], p[c])));
@@ -334,6 +362,8 @@ __global__ void __launch_bounds__(FLAT_THREADS) k_prox6_finish(ProxArgs a0, cons
                                             cabs2(csub(xb[c], x[c])));
         }
       }
+    }
+    if (NORMS) {
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         pb[c] = p[c];
