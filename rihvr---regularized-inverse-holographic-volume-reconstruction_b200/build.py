@@ -50,14 +50,15 @@ def _mtime(p: str) -> float:
 
 
 def _newest_input(path: str, seen: set) -> float:
-    """Newest of a source file and the project headers it includes."""
+    """Newest of a source file and the project headers it includes, beside it or in the public folder (-I)."""
     path = os.path.normpath(path)
     if path in seen or not os.path.exists(path):
         return -1.0
     seen.add(path)
     with open(path) as f:
         names = _INCLUDE.findall(f.read())
-    return max([_mtime(path)] + [_newest_input(os.path.join(os.path.dirname(path), n), seen) for n in names])
+    return max([_mtime(path)] + [_newest_input(os.path.join(d, n), seen)
+                                 for n in names for d in (os.path.dirname(path), INCLUDE)])
 
 
 def _compile(src: str, force: bool, verbose: bool) -> str:
