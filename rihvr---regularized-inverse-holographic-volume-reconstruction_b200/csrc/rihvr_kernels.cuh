@@ -73,6 +73,7 @@ int segment_volume(int storage, const void* P, const void* Pprev, float beta, in
                    const rihvr_segment_params* sp, rihvr_object* objects, int max_objects, int* num_objects,
                    rihvr_segment_info* info, SegWorkspace* ws, cudaStream_t st);
 size_t max_partial_blocks(int W, int H, int Nz);
+size_t prox6_partial_blocks(int W, int H, int Nz);  // of the 3-D TV prox
 
 // planes whose adjoint column pass has the recurrence variant
 bool adj_recurrence_supported(int W, int H, int rec_mode = 2);

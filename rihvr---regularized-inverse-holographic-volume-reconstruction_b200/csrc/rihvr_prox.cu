@@ -23,7 +23,9 @@ size_t max_partial_blocks(int W, int H, int Nz) {
   using Sh = TvwShape<kStripNtvMax, 2>;
   const size_t strip = (size_t)((W + Sh::VW - 1) / Sh::VW) * (size_t)std::min(64, H) * Nz;
   const size_t flat = 4096;
-  return std::max(std::max(tv, strip), flat);
+  // the 3-D TV prox's finish pass, a block a 64 x 8 tile at least: more than the
+  // others on one tall plane (4200 blocks at 588 x 3360)
+  return std::max({tv, strip, flat, prox6_partial_blocks(W, H, Nz)});
 }
 
 cudaError_t launch_prox_tv2d(int storage, const ProxArgs& a, int* nblocks_out, cudaStream_t st) {

@@ -374,21 +374,35 @@ __global__ void __launch_bounds__(FLAT_THREADS) k_prox6_finish(ProxArgs a0, cons
   block_write_sums<FLAT_THREADS>(acc, a.partials, (int)((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x));
 }
 
+// Blocks of the finish pass: 64 x 8 tiles and runs of planes, about eight blocks an SM,
+// one run of planes a block.
+struct FinishGrid {
+  int bx, by, nseg, len;  // len: planes a run
+  long long blocks() const { return (long long)bx * by * nseg; }
+};
+static FinishGrid finish_grid(int W, int H, int Nz) {
+  FinishGrid g;
+  g.bx = (W / 2 + 31) / 32;
+  g.by = (H + 7) / 8;
+  const long long tiles = (long long)g.bx * g.by;
+  const long long nseg = std::max(1LL, std::min<long long>(Nz, (8LL * num_sms() + tiles - 1) / tiles));
+  g.len = (int)((Nz + nseg - 1) / nseg);
+  g.nseg = (Nz + g.len - 1) / g.len;
+  return g;
+}
+
+size_t prox6_partial_blocks(int W, int H, int Nz) { return (size_t)finish_grid(W, H, Nz).blocks(); }
+
 template <typename ST>
 static cudaError_t prox6_finish_launch(const ProxArgs& a, const float2* Y, int* nblocks_out, cudaStream_t st) {
-  const int bx = (a.W / 2 + 31) / 32, by = (a.H + 7) / 8;
-  const long long tiles = (long long)bx * by;
-  // about eight blocks an SM; one run of planes a block
-  long long nseg = std::max(1LL, std::min<long long>(a.Nz, (8LL * num_sms() + tiles - 1) / tiles));
-  const int len = (int)((a.Nz + nseg - 1) / nseg);
-  nseg = (a.Nz + len - 1) / len;
-  const long long blocks = tiles * nseg;
-  if (by > 65535 || nseg > 65535 || blocks > a.partial_cap || blocks > 0x7fffffffLL)
+  const FinishGrid g = finish_grid(a.W, a.H, a.Nz);
+  const long long blocks = g.blocks();
+  if (g.by > 65535 || g.nseg > 65535 || blocks > a.partial_cap || blocks > 0x7fffffffLL)
     return cudaErrorInvalidConfiguration;
   *nblocks_out = (int)blocks;
-  const dim3 grid((unsigned)bx, (unsigned)by, (unsigned)nseg);
-  if (a.want_norms) k_prox6_finish<ST, true><<<grid, FLAT_THREADS, 0, st>>>(a, Y, len);
-  else k_prox6_finish<ST, false><<<grid, FLAT_THREADS, 0, st>>>(a, Y, len);
+  const dim3 grid((unsigned)g.bx, (unsigned)g.by, (unsigned)g.nseg);
+  if (a.want_norms) k_prox6_finish<ST, true><<<grid, FLAT_THREADS, 0, st>>>(a, Y, g.len);
+  else k_prox6_finish<ST, false><<<grid, FLAT_THREADS, 0, st>>>(a, Y, g.len);
   return cudaGetLastError();
 }
 
