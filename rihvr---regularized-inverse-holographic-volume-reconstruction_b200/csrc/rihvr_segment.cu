@@ -66,7 +66,14 @@ namespace seg {
 
 constexpr int kMaxClose = 15;                              // ball radius limit (shifts stay within one word)
 constexpr int kMaxRows = (2 * kMaxClose + 1) * (2 * kMaxClose + 1);
-__constant__ int c_rows[kMaxRows];                         // (dz + 64) << 16 | (dy + 64) << 8 | rx
+// The ball's rows, (dz + 64) << 16 | (dy + 64) << 8 | rx each.  A launch carries its own
+// copy as a parameter (3.8 of 4 KB), in the constant bank as a __constant__ array would
+// be: one array for the process was overwritten by the segmentation of another context
+// or thread while a kernel still read it.
+struct BallRows {
+  int n;
+  int row[kMaxRows];
+};
 constexpr int kMaxFind = 1 << 26;                          // pointer-chasing bound (error flag beyond)
 
 struct Dims {
@@ -189,9 +196,10 @@ __device__ __forceinline__ unsigned shifted(unsigned wm1, unsigned w0, unsigned 
 // rows to visit; the dilation visits only those, the erosion ends at 0 when
 // any is missing.  Rows of the output with a voxel on are flagged in row_out.
 template <bool DILATE>
-__global__ void k_morph(const unsigned* __restrict__ in, unsigned* __restrict__ out, Dims d, int nrows,
-                        const unsigned char* __restrict__ row_in, unsigned char* __restrict__ row_out) {
-  const int lane = threadIdx.x & 31;
+__global__ void k_morph(const unsigned* __restrict__ in, unsigned* __restrict__ out, Dims d,
+                        const __grid_constant__ BallRows ball, const unsigned char* __restrict__ row_in,
+                        unsigned char* __restrict__ row_out) {
+  const int lane = threadIdx.x & 31, nrows = ball.n;
   const unsigned WW = (unsigned)d.WW, Hu = (unsigned)d.H;  // 32-bit indices
   const unsigned chunks = (WW + 31) / 32;
   const unsigned ntask = (unsigned)d.H * (unsigned)d.Nz * chunks;
@@ -208,7 +216,7 @@ __global__ void k_morph(const unsigned* __restrict__ in, unsigned* __restrict__ 
       const int r = r0 + lane;
       bool live = false;
       if (r < nrows) {
-        const int e = c_rows[r];
+        const int e = ball.row[r];
         const int zz = z + (e >> 16) - 64, yy = y + ((e >> 8) & 0xff) - 64;
         live = zz >= 0 && zz < d.Nz && yy >= 0 && yy < d.H && __ldg(row_in + (unsigned)zz * Hu + yy);
       }
@@ -219,7 +227,7 @@ __global__ void k_morph(const unsigned* __restrict__ in, unsigned* __restrict__ 
         break;
       }
       for (; mask; mask &= mask - 1) {
-        const int e = c_rows[r0 + __ffs(mask) - 1];
+        const int e = ball.row[r0 + __ffs(mask) - 1];
         const int zz = z + (e >> 16) - 64, yy = y + ((e >> 8) & 0xff) - 64, rx = e & 0xff;
         if (wx >= d.WW) continue;
         const unsigned* rp = in + ((unsigned)zz * Hu + yy) * WW;
@@ -758,12 +766,13 @@ int segment_impl(SRC src, int W, int H, int Nz, const rihvr_segment_params* sp, 
   const int gw = grid_for(d.nwords, 256);
   if (sp->close_size > 0) {
     std::vector<int> rows;
-    const int nrows = ball_rows(sp->close_size, rows, &nstrel);
-    SCK(cudaMemcpyToSymbolAsync(c_rows, rows.data(), sizeof(int) * nrows, 0, cudaMemcpyHostToDevice, st));
+    BallRows ball;
+    ball.n = ball_rows(sp->close_size, rows, &nstrel);
+    std::copy(rows.begin(), rows.end(), ball.row);
     const long long mtasks = (long long)H * Nz * ((d.WW + 31) / 32);
-    k_morph<true><<<grid_for(mtasks * 32, 256), 256, 0, st>>>(bits0, bits1, d, nrows, row0, row1);
+    k_morph<true><<<grid_for(mtasks * 32, 256), 256, 0, st>>>(bits0, bits1, d, ball, row0, row1);
     SCK(cudaGetLastError());
-    k_morph<false><<<grid_for(mtasks * 32, 256), 256, 0, st>>>(bits1, bits2, d, nrows, row1, row2);
+    k_morph<false><<<grid_for(mtasks * 32, 256), 256, 0, st>>>(bits1, bits2, d, ball, row1, row2);
     SCK(cudaGetLastError());
     launches += 2;
     closed = bits2;
