@@ -213,13 +213,9 @@ template <int NT, int MT>
 cudaError_t conv3_launch(const float* X, int Cin, const __nv_bfloat16* Wt, int Cout, int co0, const float* bias,
                          float* Y, Vol v, int relu, int mirror, cudaStream_t st) {
   const size_t smem = conv_smem<MT>(NT * 8);
-  static bool opted = false;  // shared-memory opt-in, once per instantiation
-  if (!opted) {
-    const cudaError_t e = cudaFuncSetAttribute(k_conv3<NT, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem);
-    if (e != cudaSuccess) return e;
-    opted = true;
-  }
+  // the opt-in belongs to the device's context, so every launch asks for it
+  const cudaError_t e = cudaFuncSetAttribute(k_conv3<NT, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
   const unsigned blocks = (unsigned)(((v.W + kBX - 1) / kBX) * ((v.H + Brick<MT>::BY - 1) / Brick<MT>::BY) *
                                      ((v.D + kBZ - 1) / kBZ));
   k_conv3<NT, MT><<<blocks, kConvThreads, smem, st>>>(X, Cin, Wt, Cout, co0, bias, Y, v, relu, mirror);

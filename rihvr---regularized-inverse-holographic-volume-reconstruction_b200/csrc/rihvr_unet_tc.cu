@@ -279,13 +279,9 @@ template <int CN>
 cudaError_t tc_launch(const float* X, int Cin, const __nv_bfloat16* Wt, int Cout, int co0, const float* bias,
                       float* Y, int D, int H, int W, int relu, int mirror, int* err, cudaStream_t st) {
   constexpr size_t smem = tc_smem<CN>();
-  static bool opted = false;  // shared-memory opt-in, once per instantiation
-  if (!opted) {
-    const cudaError_t e = cudaFuncSetAttribute(k_conv3_tc<CN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem);
-    if (e != cudaSuccess) return e;
-    opted = true;
-  }
+  // the opt-in belongs to the device's context, so every launch asks for it
+  const cudaError_t e = cudaFuncSetAttribute(k_conv3_tc<CN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
   const unsigned blocks = (unsigned)((W / kTcX) * ((H + kTcYT - 1) / kTcYT) * D);
   k_conv3_tc<CN><<<blocks, kTcThreads, smem, st>>>(X, Cin, Wt, Cout, co0, bias, Y, D, H, W, relu, mirror, err);
   return cudaGetLastError();
@@ -779,13 +775,9 @@ cudaError_t tcb_launch(const TcMap& m, const TcMap& ms, int CinA, int Cin, const
                        const float* bias, __nv_bfloat16* Y, int D, int H, int W, const TcHead& hd, int* err,
                        cudaStream_t st) {
   constexpr size_t smem = tcb_smem<CN>();
-  static bool opted = false;
-  if (!opted) {
-    const cudaError_t e = cudaFuncSetAttribute(k_conv3_tc_bf16<CN, HEAD>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    opted = true;
-  }
+  const cudaError_t e = cudaFuncSetAttribute(k_conv3_tc_bf16<CN, HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)smem);
+  if (e != cudaSuccess) return e;
   CUtensorMap map, smap;
   static_assert(sizeof(map) == sizeof(m.bytes), "tensor map size");
   std::memcpy(&map, m.bytes, sizeof(map));
@@ -864,12 +856,8 @@ cudaError_t tcz_launch(const TcMap& m, const TcMap& skip, int CinA, const __nv_b
   constexpr int YT = S::YT;
   constexpr size_t smem = tcz_smem<CN, NS>();
   const auto kern = k_conv3_tcz<CN, HEAD, NS>;
-  static bool opted = false;
-  if (!opted) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    opted = true;
-  }
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTcThreads, smem) != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
