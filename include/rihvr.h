@@ -272,12 +272,14 @@ int rihvr_autotune(rihvr_ctx* ctx, double* best_ms);
  * plane, 1 advanced by a recurrence with the inter-stage twiddles regenerated
  * each plane, 2 the recurrence with the twiddles kept in registers (these two
  * up to side 1024, except 384 and 768), 3 the recurrence with the twiddles
- * read from a per-block shared table.  fwd_horner receives the forward column
+ * read from a per-block shared table; rectangular planes have 2 and 3.  fwd_horner receives the forward column
  * pass's variant: 1 when it sums over evenly spaced planes by Horner's scheme
  * (heights of 32 to 512 and 1024) with its input strip
  * double-buffered, 2 for the same sum with the strip staged in the exchange
  * buffer and a shared twiddle table (also sides 384, 768 and 2304), 3 for
- * that form with the strip loaded by TMA, else 0.  Any pointer may be NULL. */
+ * that form with the strip loaded by TMA, else 0; rectangular planes have 3.
+ * Both are 0 on rectangular planes narrower than a block of columns (4 to 32).
+ * Any pointer may be NULL. */
 int rihvr_tuning(const rihvr_ctx* ctx, int* adj_chunks, int* fwd_chunks, int* tv_runs, int* tv_kernel,
                  int* adj_recurrence, int* fwd_horner);
 

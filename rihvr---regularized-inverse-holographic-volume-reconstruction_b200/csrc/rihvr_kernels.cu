@@ -55,9 +55,12 @@ static cudaError_t launch_rows_fast(int inverse, int in_kind, const void* in, in
 
 bool adj_recurrence_supported(int W, int H, int rec_mode) {
   switch (H) {
-#define RIHVR_CASE(NN) \
-  case NN:             \
-    return rec_mode == 3 ? kTableCols<NN> : (kHoistTw<NN> && (NN % ColLayout<NN>::CC == 0));
+  // rectangular planes: the TMA-fed forms only, which need a column block's width (adj_col_n)
+#define RIHVR_CASE(NN)                                                                         \
+  case NN:                                                                                     \
+    return W != NN && (rec_mode == 1 || W < ColLayout<NN>::CC) ? false                         \
+           : rec_mode == 3                                     ? kTableCols<NN>                \
+                                                               : (kHoistTw<NN> && (NN % ColLayout<NN>::CC == 0));
     RIHVR_FOR_EACH_SIZE(RIHVR_CASE)
 #undef RIHVR_CASE
     default:
@@ -141,9 +144,12 @@ int adj_col_builtin(int W, int H, int Nz) {
 
 bool fwd_horner_supported(int W, int H, int horner_mode) {
   switch (H) {
-#define RIHVR_CASE(NN) \
-  case NN:             \
-    return horner_mode >= 2 ? kTableCols<NN> : (ColLayout<NN>::STAGE && LineCfg<NN>::EXACT);
+  // rectangular planes: the TMA-fed form only, which needs a column block's width (fwd_col_n)
+#define RIHVR_CASE(NN)                                                                    \
+  case NN:                                                                                \
+    return W != NN && (horner_mode != 3 || W < ColLayout<NN>::CC) ? false                 \
+           : horner_mode >= 2                                     ? kTableCols<NN>        \
+                                                                  : (ColLayout<NN>::STAGE && LineCfg<NN>::EXACT);
     RIHVR_FOR_EACH_SIZE(RIHVR_CASE)
 #undef RIHVR_CASE
     default:

@@ -75,7 +75,7 @@ int segment_volume(int storage, const void* P, const void* Pprev, float beta, in
 size_t max_partial_blocks(int W, int H, int Nz);
 size_t prox6_partial_blocks(int W, int H, int Nz);  // of the 3-D TV prox
 
-// planes whose adjoint column pass has the recurrence variant
+// planes whose adjoint column pass runs the recurrence variant `rec_mode` (launch_adj_col)
 bool adj_recurrence_supported(int W, int H, int rec_mode = 2);
 // the variant (rec_mode) the adjoint column pass takes untuned for evenly spaced planes
 int adj_col_builtin(int W, int H, int Nz);
