@@ -239,6 +239,8 @@ struct rihvr_ctx {
   cudaGraphExec_t g_mom = nullptr;
   int g_mom_n = 0;
   bool graphs = true;                // cleared when a capture fails
+  bool graphs_pay = false;           // mode 6: enough iterations asked for (expect_iterations)
+  int eager_its = 0;                 // mode 6: iterations run without graphs
   // whole iterations with the backtracking decided on the device: one graph
   // per index of P_k, kernels in [first attempt + finish/momentum, backtrack]
   cudaGraphExec_t g_iter[3] = {};
@@ -656,7 +658,23 @@ void drop_graphs(rihvr_ctx* c) {
     }
 }
 
-bool use_graphs(const rihvr_ctx* c) { return c->graphs && c->warm && !c->profiling; }
+// Capturing and instantiating a context's graphs takes 0.4 ms, once, and saves 0.02
+// to 0.03 ms an iteration of the 3-D TV solve (0.091 ms eagerly and 0.060 so at
+// 64 x 64 x 8, 0.11 and 0.083 at 128 x 128 x 32, 0.32 and 0.30 at 256 x 256 x 100).
+// A short solve on a new context does not win that back (of 5 iterations: 0.52 ms
+// eagerly, 0.78 with graphs; 0.63 and 0.90; 1.72 and 2.01), one of 20 does (1.9 and
+// 1.6; 2.3 and 2.1; 6.5 and 6.4), so mode 6 runs eagerly until a run brings a
+// context's iterations to this many.
+constexpr int kGraphIterations = 16;
+
+// `n` more iterations are asked for.
+void expect_iterations(rihvr_ctx* c, int n) {
+  if (n + c->eager_its >= kGraphIterations) c->graphs_pay = true;
+}
+
+bool use_graphs(const rihvr_ctx* c) {
+  return c->graphs && c->warm && !c->profiling && (c->mode != 6 || c->graphs_pay);
+}
 
 // Run `enqueue` as a CUDA graph (captured on first use) or eagerly.  A failed
 // capture turns graphs off for the context and runs the work eagerly.
@@ -1281,6 +1299,7 @@ int one_iteration(rihvr_ctx* c) {
   c->pending_x = (int)c->log.size() - 1;
   c->it++;
   c->warm = true;
+  if (!c->graphs_pay) ++c->eager_its;
   return RIHVR_OK;
 }
 
@@ -1299,6 +1318,7 @@ int settle_pending(rihvr_ctx* c) {
 
 // Iterations i .. n-1 of a run, after the eager first one (when it ran).
 int run_iterations_from(rihvr_ctx* c, int i, int n) {
+  expect_iterations(c, n - i);
   if (i < n && use_dev_loop(c)) {
     if (ensure_iter_graphs(c) == RIHVR_OK) {
       RC(run_iterations_dev(c, n - i));
@@ -1319,6 +1339,7 @@ int eager_start(rihvr_ctx* c, int n, int* ran) {
     RC(one_iteration(c));
     *ran = 1;
   }
+  expect_iterations(c, n - *ran);
   return RIHVR_OK;
 }
 
