@@ -1526,12 +1526,16 @@ int create_ctx(const rihvr_params* params, int width, int height, int z_first, i
   c->nchunks = fwd_col_chunks(width, height, c->Nz);
   if (rc == RIHVR_OK) rc = dalloc_t(c, &c->Spart, c->HW * kMaxFwdChunks);
   if (rc == RIHVR_OK) rc = dalloc_t(c, &c->S, c->HW);
-  if (rc == RIHVR_OK) rc = dalloc_t(c, &c->pc1, c->HW);
-  if (rc == RIHVR_OK) rc = dalloc_t(c, &c->pc2, c->HW);
-  if (rc == RIHVR_OK) rc = dalloc_t(c, &c->Rs, c->HW);
-  for (float2** q : {&c->Bh, &c->Dn, &c->D0, &c->DX})
-    if (rc == RIHVR_OK) rc = dalloc_t(c, q, c->HW);
-  if (rc == RIHVR_OK) rc = dalloc_t(c, &c->block_count, 1);
+  // the complex planes, 256 bytes apart, in one allocation (one each took a
+  // tenth of a context's creation at 640 x 640 x 150)
+  float2** const cplanes[] = {&c->pc1, &c->pc2, &c->Rs, &c->Bh, &c->Dn, &c->D0, &c->DX};
+  const size_t pitch = (c->HW + 31) / 32 * 32, ncp = std::size(cplanes);
+  float2* cplane = nullptr;
+  if (rc == RIHVR_OK) rc = dalloc_t(c, &cplane, ncp * pitch + 1);
+  if (rc == RIHVR_OK) {
+    for (size_t i = 0; i < ncp; ++i) *cplanes[i] = cplane + i * pitch;
+    c->block_count = reinterpret_cast<unsigned*>(cplane + ncp * pitch);
+  }
   if (rc == RIHVR_OK) rc = dalloc_t(c, &c->b, c->HW);
   if (rc == RIHVR_OK) rc = dalloc_t(c, &c->dnew, c->HW);
   if (rc == RIHVR_OK) rc = dalloc_t(c, &c->dY0, c->HW);
