@@ -34,7 +34,7 @@ HOST_CXX = shutil.which("g++") or "g++"
 
 LIB_SOURCES = ["rihvr_fast_small.cu", "rihvr_fast_mid.cu", "rihvr_fast_640.cu", "rihvr_fast_large.cu",
                "rihvr_kernels.cu", "rihvr_prox.cu", "rihvr_prox_f32.cu", "rihvr_prox_f16.cu",
-               "rihvr_prox_bf16.cu", "rihvr_lines.cu", "rihvr_lines_long.cu", "rihvr_tv3d.cu",
+               "rihvr_prox_bf16.cu", "rihvr_lines.cu", "rihvr_lines_long.cu", "rihvr_plane64.cu", "rihvr_tv3d.cu",
                "rihvr_solver.cu", "rihvr_params.cpp", "rihvr_noalloc.cu", "rihvr_image.cpp",
                "rihvr_segment.cu", "rihvr_unet.cu", "rihvr_unet_tc.cu",
                "rihvr_unet_grad.cu", "rihvr_frame.cu"]

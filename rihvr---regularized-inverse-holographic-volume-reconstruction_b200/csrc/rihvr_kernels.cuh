@@ -119,6 +119,8 @@ cudaError_t launch_reduce_partials(const double* partials, int nblocks, double* 
 size_t reduce_scratch_doubles();
 constexpr int kReduceOneLaunch = 2048;  // block partials summed by one launch; more take two
 cudaError_t launch_fill_uniform_c(float2* x, long long n, unsigned long long seed, cudaStream_t st);
+// dst = FFT2(src) of a real plane, in FP64 rounded once; work: W x H double2
+cudaError_t launch_plane_spectrum(const float* src, double2* work, float2* dst, int W, int H, cudaStream_t st);
 cudaError_t launch_sumsq(const float* x, long long n, double* partials, int* nblocks_out, cudaStream_t st);
 cudaError_t launch_finish_forward(const float2* c, const float* b, float* dnew, long long n, double* partials,
                                   int* nblocks_out, cudaStream_t st);

@@ -405,11 +405,12 @@ SpecSums spec_sums(const rihvr_ctx* c, int slot) {
   return SpecSums{c->partials, c->sums_d + slot * kNumSums, c->block_count};
 }
 
-// dst = spectrum of the real plane src (exactly Hermitian)
+// dst = spectrum of the real plane src (exactly Hermitian), transformed in FP64
 int plane_spectrum(rihvr_ctx* c, const float* src, float2* dst) {
   ProfScope ps(c, K_PLANE);
-  KL(launch_rows(0, ELEM_R32, src, ELEM_C32, c->pc1, c->W, c->H, 1.0f, c->st));
-  KL(launch_plane_col(0, c->pc1, c->pc2, c->W, c->H, 1.0f, c->st));
+  static_assert(kMaxFwdChunks >= 2, "the chunks' sums leave room for a plane of double2");
+  KL(launch_plane_spectrum(src, reinterpret_cast<double2*>(c->Spart), c->pc2, c->W, c->H, c->st));
+  ++c->launches;  // a row and a column pass
   KL(launch_spec_residual(c->pc2, 1, nullptr, dst, c->W, c->H, spec_sums(c, SLOT_FWD), c->st));
   return RIHVR_OK;
 }
@@ -588,7 +589,6 @@ int state_reset(rihvr_ctx* c) {
   c->log.clear();
   c->pending_x = -1;
   // x = 0: d = 0, r = -b (:273)
-  RC(plane_spectrum(c, c->b, c->Bh));
   for (float2* q : {c->Dn, c->D0}) CK(cudaMemsetAsync(q, 0, sizeof(float2) * c->HW, c->st));
   RC(momentum_spectrum(c, 0.f));
   int nb = 0;
@@ -1489,6 +1489,17 @@ int rihvr_debug_fail_allocations_after(int n) { return g_alloc_budget.exchange(n
 
 namespace {
 
+// The measured hologram b (checked), its spectrum and the state x = 0.
+int take_hologram(rihvr_ctx* c, const float* b, int is_device) {
+  c->have_holo = false;  // until both are the new one's
+  RC(copy_in(c, c->b, b, sizeof(float) * c->HW, is_device));
+  RC(plane_spectrum(c, c->b, c->Bh));
+  c->have_holo = true;
+  RC(state_reset(c));
+  if (c->p.autotune && !c->tuned) RC(rihvr_autotune(c, nullptr));
+  return RIHVR_OK;
+}
+
 // A context for planes [z_first, z_first + z_count) of the plane list
 // (all of them for rihvr_create); params and sizes already validated.
 int create_ctx(const rihvr_params* params, int width, int height, int z_first, int z_count, rihvr_ctx** out) {
@@ -1650,11 +1661,7 @@ int rihvr_set_hologram(rihvr_ctx* c, const float* b, int is_device) {
   }
   if (bad)
     return fail(RIHVR_ERR_INVALID_DATA, "hologram has " + std::to_string(bad) + " non-finite samples");
-  RC(copy_in(c, c->b, b, sizeof(float) * c->HW, is_device));
-  c->have_holo = true;
-  RC(state_reset(c));
-  if (c->p.autotune && !c->tuned) RC(rihvr_autotune(c, nullptr));
-  return RIHVR_OK;
+  return take_hologram(c, b, is_device);
 }
 
 int rihvr_set_hologram_frame(rihvr_ctx* c, const void* frame, int bits, int width, int height,
@@ -1665,11 +1672,7 @@ int rihvr_set_hologram_frame(rihvr_ctx* c, const void* frame, int bits, int widt
   // state change only when that succeeded
   RC(frame_to_hologram(&c->frame_ws, frame, bits, width, height, background, files, c->p.zero_padding, c->W, c->H,
                        is_device, c->st, &staged, &c->launches));
-  RC(copy_in(c, c->b, staged, sizeof(float) * c->HW, 1));
-  c->have_holo = true;
-  RC(state_reset(c));
-  if (c->p.autotune && !c->tuned) RC(rihvr_autotune(c, nullptr));
-  return RIHVR_OK;
+  return take_hologram(c, staged, 1);
 }
 
 int rihvr_get_hologram(rihvr_ctx* c, float* out, int is_device) {
