@@ -485,6 +485,23 @@ __device__ __forceinline__ float2 transfer_accurate(double z, double cturn, bool
   return make_float2(c, conj_ ? -s : s);
 }
 
+// What Horner's sum over planes 0 .. n with the rotation d (D = H'_dz in FP32) is
+// multiplied by: H'_z of its first plane, turned by what d^(n/2) has drifted from
+// D^(n/2), so that term k carries the drift of |k - n/2| steps instead of k.  `drift`
+// holds D / d - 1 (HornerTable); left out where a chunk has too few planes to drift by
+// an ulp.  512 x 512 x 100, 17 planes a chunk: 4.1e-7 from the exact sum with d from a
+// phase rounded to FP32 and no drift, 3.2e-7 so; the volume of a solve at 1024 x 1024 x
+// 1000, 200 planes a chunk: 1.6e-6 and 4.3e-7.
+constexpr int kHornerDrift = 8;
+template <bool DRIFT>
+__device__ __forceinline__ float2 horner_anchor(double z, double cturn, const __half2* drift, int n) {
+  const float2 h = transfer_accurate(z, cturn, false);
+  if (!DRIFT) return h;
+  const float2 e = __half22float2(__ldg(drift));
+  return cadd(h, cmul(h, cscale(e, 0.5f * (float)n / kHornerDriftScale)));
+}
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // Planes between exact re-anchorings of the adjoint recurrence.  FP32
 // rotations drift by about one rounding a step; 16 steps keep that near 1e-6.
 constexpr int kAdjAnchor = 16;
@@ -694,11 +711,12 @@ __global__ void __launch_bounds__(ColLayout<N>::THREADS) k_fwd_col(const float2*
 // place of the FP64 phase-table strip) instead of an FP64 phase reduction, a
 // sincos and a multiply-add; H'_{zb} is applied once, exactly, at the end.  The
 // planes go in descending order.  D^k carries the rounding of D k times (about
-// k x 6e-8 in phase), which stays near 1e-5 for the longest z-chunks used.
+// k x 2e-8 in phase); horner_anchor halves it.
 template <int N>
 __global__ void __launch_bounds__(ColLayout<N>::THREADS) k_fwd_col_horner(const float2* __restrict__ T,
                                                                           const double* __restrict__ cturn,
-                                                                          const double* __restrict__ zlist, double dz,
+                                                                          const double* __restrict__ zlist,
+                                                                          const HornerTable table,
                                                                           float2* __restrict__ Spart, int z0, int z1,
                                                                           int zpb) {
   constexpr int W = N;  // square planes
@@ -714,6 +732,7 @@ __global__ void __launch_bounds__(ColLayout<N>::THREADS) k_fwd_col_horner(const 
   const int zb = z0 + blockIdx.y * zpb, ze = min(zb + zpb, z1);
   const size_t HW = (size_t)N * W;
   const double* ct = cturn + (size_t)t * W + x;
+  const float2* rot = table.d + (size_t)t * W + x;
   float2* const s_t = sm + Lay::SMEM_ELEMS;       // one strip of T
   float2* const s_d = s_t + Lay::STRIP_ELEMS;     // this thread's rotations D, stage-B layout
   if (zb < ze) strip_async<N>(s_t, T + (size_t)(ze - 1) * HW, blockIdx.x * CC, W);
@@ -722,7 +741,7 @@ __global__ void __launch_bounds__(ColLayout<N>::THREADS) k_fwd_col_horner(const 
   for (int j = 0; j < M; ++j)
 #pragma unroll
     for (int k1 = 0; k1 < N1; ++k1)
-      s_d[(N1 * j + N2 * k1 + t) * CC + c] = transfer_accurate(dz, __ldg(ct + (size_t)(N1 * j + N2 * k1) * W), false);
+      s_d[(N1 * j + N2 * k1 + t) * CC + c] = __ldg(rot + (size_t)(N1 * j + N2 * k1) * W);
   float2 acc[N2];
 #pragma unroll
   for (int i = 0; i < N2; ++i) acc[i] = make_float2(0.f, 0.f);
@@ -756,14 +775,20 @@ __global__ void __launch_bounds__(ColLayout<N>::THREADS) k_fwd_col_horner(const 
   cp_async_wait<0>();
   if (col_ok && zb < ze) {
     const double zz = zlist[zb];
+    const int We = W;
     float2* Sp = Spart + (size_t)blockIdx.y * HW + (size_t)t * W + x;
+    const __half2* dr = table.drift + (size_t)t * W + x;
+    const auto finish = [&](auto with) {  // one test for the chunk: the loads of all elements can be in flight
 #pragma unroll
-    for (int j = 0; j < M; ++j)
+      for (int j = 0; j < M; ++j)
 #pragma unroll
-      for (int k1 = 0; k1 < N1; ++k1) {
-        const float2 h = transfer_accurate(zz, __ldg(ct + (size_t)(N1 * j + N2 * k1) * W), false);
-        Sp[(size_t)(N1 * j + N2 * k1) * W] = cmul(acc[j * N1 + k1], h);
-      }
+        for (int k1 = 0; k1 < N1; ++k1) {
+          const size_t o = (size_t)(N1 * j + N2 * k1) * We;
+          Sp[o] = cmul(acc[j * N1 + k1], horner_anchor<decltype(with)::value>(zz, __ldg(ct + o), dr + o, ze - 1 - zb));
+        }
+    };
+    if (ze - 1 - zb < kHornerDrift) finish(std::false_type{});
+    else finish(std::true_type{});
   } else if (col_ok) {
     float2* Sp = Spart + (size_t)blockIdx.y * HW + (size_t)t * W + x;
 #pragma unroll
@@ -844,8 +869,9 @@ __device__ __forceinline__ void tma_load_3d(void* smem, const CUtensorMap* map, 
 template <int N, bool TMA, bool SQ>
 __global__ void __launch_bounds__(ColLayout<N>::THREADS, col3_minb<N>())
     k_fwd_col_horner1(const float2* __restrict__ T, const double* __restrict__ cturn,
-                      const double* __restrict__ zlist, double dz, float2* __restrict__ Spart, int z0, int z1,
-                      int zpb, int Wr, const __grid_constant__ CUtensorMap tmap, unsigned* timeouts) {
+                      const double* __restrict__ zlist, const HornerTable table,
+                      float2* __restrict__ Spart, int z0, int z1, int zpb, int Wr,
+                      const __grid_constant__ CUtensorMap tmap, unsigned* timeouts) {
   const int W = SQ ? N : Wr;
   using C = LineCfg<N>;
   using Lay = ColLayout<N>;
@@ -860,6 +886,7 @@ __global__ void __launch_bounds__(ColLayout<N>::THREADS, col3_minb<N>())
   const int zb = z0 + blockIdx.y * zpb, ze = min(zb + zpb, z1);
   const size_t HW = (size_t)N * W;
   const double* ct = cturn + (size_t)t * W + x;
+  const float2* rot = table.d + (size_t)t * W + x;
   float2* const s_d = sm + BUF;                  // this thread's rotations D, stage-B layout
   float2* const s_tw = s_d + Lay::STRIP_ELEMS;   // twiddle table
   uint64_t* const bar = reinterpret_cast<uint64_t*>(s_tw + TwTable<N>::ELEMS);
@@ -894,7 +921,12 @@ __global__ void __launch_bounds__(ColLayout<N>::THREADS, col3_minb<N>())
   for (int j = 0; j < M; ++j)
 #pragma unroll
     for (int k1 = 0; k1 < N1; ++k1)
-      s_d[(N1 * j + N2 * k1 + t) * CC + c] = transfer_accurate(dz, __ldg(ct + (size_t)(N1 * j + N2 * k1) * W), false);
+      s_d[(N1 * j + N2 * k1 + t) * CC + c] = __ldg(rot + (size_t)(N1 * j + N2 * k1) * W);
+  {  // the phases are next read at the end, by all blocks of a wave at once
+    const int Wp = SQ ? N : launder_i(Wr);
+#pragma unroll
+    for (int i = 0; i < N; i += N1) prefetch_l2(ct + (size_t)i * Wp);
+  }
   float2 acc[N2];
 #pragma unroll
   for (int i = 0; i < N2; ++i) acc[i] = make_float2(0.f, 0.f);
@@ -945,14 +977,20 @@ __global__ void __launch_bounds__(ColLayout<N>::THREADS, col3_minb<N>())
   if constexpr (!TMA) cp_async_wait<0>();
   if (col_ok && zb < ze) {
     const double zz = zlist[zb];
+    const int We = SQ ? N : launder_i(Wr);  // own row offsets: kept from the start, they would take the sums' registers
     float2* Sp = Spart + (size_t)blockIdx.y * HW + (size_t)t * W + x;
+    const __half2* dr = table.drift + (size_t)t * W + x;
+    const auto finish = [&](auto with) {  // one test for the chunk: the loads of all elements can be in flight
 #pragma unroll
-    for (int j = 0; j < M; ++j)
+      for (int j = 0; j < M; ++j)
 #pragma unroll
-      for (int k1 = 0; k1 < N1; ++k1) {
-        const float2 h = transfer_accurate(zz, __ldg(ct + (size_t)(N1 * j + N2 * k1) * W), false);
-        Sp[(size_t)(N1 * j + N2 * k1) * W] = cmul(acc[j * N1 + k1], h);
-      }
+        for (int k1 = 0; k1 < N1; ++k1) {
+          const size_t o = (size_t)(N1 * j + N2 * k1) * We;
+          Sp[o] = cmul(acc[j * N1 + k1], horner_anchor<decltype(with)::value>(zz, __ldg(ct + o), dr + o, ze - 1 - zb));
+        }
+    };
+    if (ze - 1 - zb < kHornerDrift) finish(std::false_type{});
+    else finish(std::true_type{});
   } else if (col_ok) {
     float2* Sp = Spart + (size_t)blockIdx.y * HW + (size_t)t * W + x;
 #pragma unroll
@@ -1089,20 +1127,22 @@ cudaError_t adj_col_n(const float2* Rs, const double* cturn, const double* zlist
 
 template <int N>
 cudaError_t fwd_col_n(const float2* T, const double* cturn, const double* zlist, float2* Spart, int W,
-                             int z0, int z1, int nchunks, cudaStream_t st, double dz_uniform, int horner_mode) {
+                             int z0, int z1, int nchunks, cudaStream_t st, int horner_mode,
+                             const HornerTable& table) {
   using Lay = ColLayout<N>;
   const int nz = z1 - z0;
   if (nz <= 0) return cudaSuccess;
   const int strips = col_strips<N>(W);
   const int zpb = (nz + nchunks - 1) / nchunks;
   const int chunks = (nz + zpb - 1) / zpb;
+  const bool horner = horner_mode != 0 && table.d;
   cudaError_t e;
   if (chunks < nchunks) {  // unused chunk slots must read as zero
     e = cudaMemsetAsync(Spart + (size_t)chunks * N * W, 0, sizeof(float2) * (size_t)(nchunks - chunks) * N * W, st);
     if (e != cudaSuccess) return e;
   }
   if constexpr (kTableCols<N>) {
-    if (dz_uniform != 0.0 && (horner_mode == 2 || horner_mode == 3)) {
+    if (horner && (horner_mode == 2 || horner_mode == 3)) {
       constexpr size_t smem = horner1_smem<N>();
       CUtensorMap tmap;
       std::memset(&tmap, 0, sizeof(tmap));
@@ -1114,7 +1154,7 @@ cudaError_t fwd_col_n(const float2* T, const double* cturn, const double* zlist,
         if (e2 != cudaSuccess) return e2;
         unsigned* const timeouts = col_timeout_counter();
         if (!timeouts) return cudaErrorUnknown;
-        kern<<<dim3(strips, chunks), Lay::THREADS, smem, st>>>(T, cturn, zlist, dz_uniform, Spart, z0, z1, zpb, W, tmap,
+        kern<<<dim3(strips, chunks), Lay::THREADS, smem, st>>>(T, cturn, zlist, table, Spart, z0, z1, zpb, W, tmap,
                                                                timeouts);
         return cudaGetLastError();
       };
@@ -1123,10 +1163,10 @@ cudaError_t fwd_col_n(const float2* T, const double* cturn, const double* zlist,
     }
   }
   if constexpr (Lay::STAGE && LineCfg<N>::EXACT) {
-    if (dz_uniform != 0.0 && W == N) {
+    if (horner && W == N) {
       e = allow_smem(k_fwd_col_horner<N>, Lay::STAGE_BYTES);
       if (e != cudaSuccess) return e;
-      k_fwd_col_horner<N><<<dim3(strips, chunks), Lay::THREADS, Lay::STAGE_BYTES, st>>>(T, cturn, zlist, dz_uniform,
+      k_fwd_col_horner<N><<<dim3(strips, chunks), Lay::THREADS, Lay::STAGE_BYTES, st>>>(T, cturn, zlist, table,
                                                                                          Spart, z0, z1, zpb);
       return cudaGetLastError();
     }
@@ -1161,7 +1201,7 @@ cudaError_t plane_col_n(int inverse, const float2* in, float2* out, int W, float
   LINKAGE template cudaError_t adj_col_n<NN>(const float2*, const double*, const double*, float2*, int, int, int,   \
                                              cudaStream_t, int, double, int);                                      \
   LINKAGE template cudaError_t fwd_col_n<NN>(const float2*, const double*, const double*, float2*, int, int, int,   \
-                                             int, cudaStream_t, double, int);                                      \
+                                             int, cudaStream_t, int, const HornerTable&);                          \
   LINKAGE template cudaError_t plane_col_n<NN>(int, const float2*, float2*, int, float, cudaStream_t);
 
 }  // namespace rihvr

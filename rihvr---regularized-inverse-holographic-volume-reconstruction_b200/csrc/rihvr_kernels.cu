@@ -158,17 +158,39 @@ bool fwd_horner_supported(int W, int H, int horner_mode) {
 }
 
 static cudaError_t launch_fwd_col_fast(const float2* T, const double* cturn, const double* zlist, float2* Spart,
-                                      int W, int H, int z0, int z1, int nchunks, cudaStream_t st, double dz_uniform,
-                                      int horner_mode) {
+                                      int W, int H, int z0, int z1, int nchunks, cudaStream_t st, int horner_mode,
+                                      const HornerTable& table) {
   switch (H) {
 #define RIHVR_CASE(NN) \
   case NN:             \
-    return fwd_col_n<NN>(T, cturn, zlist, Spart, W, z0, z1, nchunks, st, dz_uniform, horner_mode);
+    return fwd_col_n<NN>(T, cturn, zlist, Spart, W, z0, z1, nchunks, st, horner_mode, table);
     RIHVR_FOR_EACH_SIZE(RIHVR_CASE)
 #undef RIHVR_CASE
     default:
       return cudaErrorInvalidValue;
   }
+}
+
+// HornerTable of the spacing dz: d is D = H'_dz rounded to FP32, drift D / d - 1 times
+// kHornerDriftScale
+__global__ void __launch_bounds__(FLAT_THREADS) k_horner_table(const double* __restrict__ cturn, double dz,
+                                                               float2* __restrict__ d, __half2* __restrict__ drift,
+                                                               long long n) {
+  for (long long i = (long long)blockIdx.x * FLAT_THREADS + threadIdx.x; i < n; i += (long long)gridDim.x * FLAT_THREADS) {
+    double u = dz * cturn[i], s, c;
+    u -= rint(u);
+    sincospi(2.0 * u, &s, &c);
+    const float2 r = make_float2((float)c, (float)s);
+    const float2 e = cmulc(make_float2((float)(c - (double)r.x), (float)(s - (double)r.y)), r);  // |r| = 1
+    d[i] = r;
+    drift[i] = __float22half2_rn(cscale(e, kHornerDriftScale));
+  }
+}
+
+cudaError_t launch_horner_table(const double* cturn, double dz, float2* d, __half2* drift, long long n,
+                                cudaStream_t st) {
+  k_horner_table<<<flat_blocks((size_t)n), FLAT_THREADS, 0, st>>>(cturn, dz, d, drift, n);
+  return cudaGetLastError();
 }
 
 static cudaError_t launch_plane_col_fast(int inverse, const float2* in, float2* out, int W, int H, float scale,
@@ -638,9 +660,9 @@ cudaError_t col_wait_timeouts(cudaStream_t st, unsigned* count) {
 }
 
 cudaError_t launch_fwd_col(const float2* T, const double* cturn, const double* zlist, float2* Spart, int W, int H,
-                           int z0, int z1, int nchunks, cudaStream_t st, double dz_uniform, int horner_mode) {
+                           int z0, int z1, int nchunks, cudaStream_t st, int horner_mode, const HornerTable& table) {
   return line_size_supported(H)
-             ? launch_fwd_col_fast(T, cturn, zlist, Spart, W, H, z0, z1, nchunks, st, dz_uniform, horner_mode)
+             ? launch_fwd_col_fast(T, cturn, zlist, Spart, W, H, z0, z1, nchunks, st, horner_mode, table)
              : launch_line_fwd_col(T, cturn, zlist, Spart, W, H, z0, z1, nchunks, st);
 }
 

@@ -1,5 +1,6 @@
 // Kernel launchers shared by the solver (all asynchronous on the given stream).
 #pragma once
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -90,14 +91,23 @@ cudaError_t launch_adj_col(const float2* Rs, const double* cturn, const double* 
                            int rec_mode = 0);
 cudaError_t launch_rows(int inverse, int in_kind, const void* in, int out_kind, void* out, int W,
                         long long nlines, float scale, cudaStream_t st);
-// dz_uniform != 0 (evenly spaced planes): staged heights sum over z by
-// Horner's scheme with the rotation H'_dz (fwd_horner_supported); horner_mode
+// The rotation H'_dz from plane to plane of evenly spaced planes in FP32, for every
+// frequency (W x H), and what it loses (kHornerDriftScale times)
+struct HornerTable {
+  const float2* d = nullptr;
+  const __half2* drift = nullptr;
+};
+constexpr float kHornerDriftScale = 16777216.f;  // 2^24: of order 1 in FP16
+cudaError_t launch_horner_table(const double* cturn, double dz, float2* d, __half2* drift, long long n,
+                                cudaStream_t st);
+// With a table (evenly spaced planes) and horner_mode != 0, staged heights sum over z
+// by Horner's scheme with that rotation (fwd_horner_supported); horner_mode
 // 1 stages T in its own double buffer (two blocks an SM), 2 in the exchange
 // buffer with the twiddles in a shared table (three blocks an SM), 3 the same
 // with each strip loaded by TMA (bounded mbarrier waits, col_wait_timeouts).
 cudaError_t launch_fwd_col(const float2* T, const double* cturn, const double* zlist, float2* Spart, int W,
-                           int H, int z0, int z1, int nchunks, cudaStream_t st, double dz_uniform = 0.0,
-                           int horner_mode = 1);
+                           int H, int z0, int z1, int nchunks, cudaStream_t st, int horner_mode,
+                           const HornerTable& table);
 bool fwd_horner_supported(int W, int H, int horner_mode = 1);
 // Bounded waits of the TMA-fed column passes that ran out since the last call
 // (synchronises the stream; clears the count).  Nonzero means a forward sum

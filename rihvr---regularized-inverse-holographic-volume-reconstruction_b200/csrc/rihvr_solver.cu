@@ -213,6 +213,7 @@ struct rihvr_ctx {
   float* r = nullptr;
   double* cturn = nullptr;
   double* zlist = nullptr;
+  HornerTable horner;     // of the forward pass, where the planes are evenly spaced and the sides have its Horner sums
   double dz_uniform = 0;  // plane spacing when every z_{k+1} - z_k is the same (FP64), else 0
   // column-pass variants for evenly spaced planes (need dz_uniform): the
   // adjoint's transfer function by recurrence (1: twiddles regenerated each
@@ -466,7 +467,7 @@ int forward_chunks(rihvr_ctx* c, int kind, const void* vol) {
     const int hor = env_variant("RIHVR_FWD_COL", {"direct", "horner", "horner_onebuf", "horner_tma"},
                                 c->tune_fwd_horner);
     KL(launch_fwd_col(c->U, c->cturn, c->zlist, c->Spart, c->W, c->H, 0, c->Nz, c->nchunks, c->st,
-                      hor ? c->dz_uniform : 0.0, hor));
+                      hor, c->horner));
   }
   return RIHVR_OK;
 }
@@ -1542,7 +1543,7 @@ int create_ctx(const rihvr_params* params, int width, int height, int z_first, i
   float2** const cplanes[] = {&c->pc1, &c->pc2, &c->Rs, &c->Bh, &c->Dn, &c->D0, &c->DX};
   const size_t pitch = (c->HW + 31) / 32 * 32, ncp = std::size(cplanes);
   float2* cplane = nullptr;
-  if (rc == RIHVR_OK) rc = dalloc_t(c, &cplane, ncp * pitch + 1);
+  if (rc == RIHVR_OK) rc = dalloc_t(c, &cplane, (ncp + 1) * pitch + 32 + pitch / 2);
   if (rc == RIHVR_OK) {
     for (size_t i = 0; i < ncp; ++i) *cplanes[i] = cplane + i * pitch;
     c->block_count = reinterpret_cast<unsigned*>(cplane + ncp * pitch);
@@ -1586,11 +1587,20 @@ int create_ctx(const rihvr_params* params, int width, int height, int z_first, i
   for (int k = 1; k + 1 < c->Nz && c->dz_uniform != 0; ++k)
     if (zl[(size_t)k + 1] - zl[(size_t)k] != c->dz_uniform) c->dz_uniform = 0;
   if (c->dz_uniform != 0) c->tune_adj_rec = adj_col_builtin(width, height, c->Nz);
-  if (cudaMemcpy(c->cturn, ct.data(), sizeof(double) * ct.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(c->zlist, zl.data(), sizeof(double) * zl.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+  // on the context's stream, which does not wait for the default one
+  if (cudaMemcpyAsync(c->cturn, ct.data(), sizeof(double) * ct.size(), cudaMemcpyHostToDevice, c->st) != cudaSuccess ||
+      cudaMemcpyAsync(c->zlist, zl.data(), sizeof(double) * zl.size(), cudaMemcpyHostToDevice, c->st) != cudaSuccess ||
       cudaMemsetAsync(c->block_count, 0, sizeof(unsigned), c->st) != cudaSuccess ||
       cudaMemsetAsync(c->b, 0, sizeof(float) * c->HW, c->st) != cudaSuccess)
     return cleanup(fail(RIHVR_ERR_CUDA, "initial copies failed"));
+  if (c->dz_uniform != 0 && (fwd_horner_supported(width, height, 1) || fwd_horner_supported(width, height, 3))) {
+    float2* const d = cplane + ncp * pitch + 32;
+    __half2* const drift = reinterpret_cast<__half2*>(d + pitch);
+    if (launch_horner_table(c->cturn, c->dz_uniform, d, drift, (long long)c->HW, c->st) != cudaSuccess)
+      return cleanup(fail(RIHVR_ERR_CUDA, "launch_horner_table failed"));
+    c->horner = HornerTable{d, drift};
+  }
+  if (cudaStreamSynchronize(c->st) != cudaSuccess) return cleanup(fail(RIHVR_ERR_CUDA, "initial copies failed"));
   *out = c;
   return RIHVR_OK;
 }
@@ -1783,7 +1793,7 @@ int autotune_run(rihvr_ctx* c, cudaEvent_t e0, cudaEvent_t e1, TuneVal* out) {
       if (ch > c->Nz || ch > kMaxFwdChunks) continue;
       RC(time_min(c, e0, e1, [&]() -> int {
         KL(launch_fwd_col(c->U, c->cturn, c->zlist, c->Spart, c->W, c->H, 0, c->Nz, ch, c->st,
-                          hor ? c->dz_uniform : 0.0, hor));
+                          hor, c->horner));
         KL(launch_sum_chunks(c->Spart, ch, c->S, (long long)c->HW, c->st));
         return RIHVR_OK;
       }, &best));
