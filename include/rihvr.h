@@ -152,9 +152,11 @@ int rihvr_create(const rihvr_params* params, int width, int height, rihvr_ctx** 
 void rihvr_destroy(rihvr_ctx* ctx);
 
 /* Testing hook, no counterpart in the reference: once n more device or pinned
- * host allocations of rihvr_create have succeeded, the next one fails as if
- * memory were exhausted (RIHVR_ERR_OUT_OF_MEMORY), so that a test can walk
- * every cleanup path of rihvr_create without exhausting a GPU.  n < 0 (the
+ * host allocations of rihvr_create and of the segmentation's workspace have
+ * succeeded, the next one fails as if memory were exhausted
+ * (RIHVR_ERR_OUT_OF_MEMORY), so that a test can walk every cleanup path of
+ * rihvr_create, and the segmentation's smaller workspace, without exhausting a
+ * GPU.  n < 0 (the
  * default) turns the injection off.  Process-wide; returns the previous
  * setting. */
 int rihvr_debug_fail_allocations_after(int n);

@@ -60,6 +60,8 @@ bool line_size_supported(int n);
 bool generic_size_supported(int n);
 // message returned by rihvr_last_error on this thread
 void set_last_error(const char* msg);
+// does rihvr_debug_fail_allocations_after make this allocation fail?
+bool injected_alloc_failure();
 
 // particle segmentation of the volume x = P + beta (P - Pprev) on stream st,
 // with device buffers kept in a workspace between calls (rihvr_segment.cu)

@@ -563,6 +563,7 @@ struct SegWorkspace {
   static constexpr int kSteps = 3;
   unsigned char* p[kSteps] = {};
   size_t cap[kSteps] = {};
+  bool spare_fits = true;  // the first step's spare room; asked for once
   ~SegWorkspace() {
     for (void* q : p)
       if (q) cudaFree(q);
@@ -573,7 +574,7 @@ struct SegWorkspace {
     p[step] = nullptr;
     cap[step] = 0;
     void* q = nullptr;
-    const cudaError_t e = cudaMalloc(&q, bytes);
+    const cudaError_t e = injected_alloc_failure() ? cudaErrorMemoryAllocation : cudaMalloc(&q, bytes);
     if (e != cudaSuccess) return e;
     p[step] = static_cast<unsigned char*>(q);
     cap[step] = bytes;
@@ -690,11 +691,12 @@ int segment_impl(SRC src, int W, int H, int Nz, const rihvr_segment_params* sp, 
   const size_t o_q = kStoreQ ? c0.add<float>((size_t)nvox) : 0;
   // room for the later steps when few voxels are on, as particles have it (one
   // in 200; about 52 bytes each), so that a call allocates once
-  size_t spare = 65536 + (size_t)nvox / 4;
+  size_t spare = ws.spare_fits ? 65536 + (size_t)nvox / 4 : 0;
   const size_t without = c0.bytes, o_spare = c0.add<unsigned char>(spare);
-  cudaError_t e0 = ws.reserve(0, c0.bytes);
-  if (e0 == cudaErrorMemoryAllocation) {  // the steps then allocate their own
+  cudaError_t e0 = ws.reserve(0, spare > 0 ? c0.bytes : without);
+  if (e0 == cudaErrorMemoryAllocation && spare > 0) {  // the steps then allocate their own, in later calls too
     cudaGetLastError();
+    ws.spare_fits = false;
     spare = 0;
     e0 = ws.reserve(0, without);
   }

@@ -289,13 +289,17 @@ namespace {
 // succeed; the one after them fails as if the device were out of memory.
 std::atomic<int> g_alloc_budget{-1};
 
-bool injected_alloc_failure() {
+}  // namespace
+
+bool rihvr::injected_alloc_failure() {
   int b = g_alloc_budget.load();
   while (b >= 0) {
     if (g_alloc_budget.compare_exchange_weak(b, b - 1)) return b == 0;
   }
   return false;
 }
+
+namespace {
 
 int dalloc(rihvr_ctx* c, void** p, size_t n) {
   if (injected_alloc_failure()) {
