@@ -9,8 +9,10 @@
 //
 // A block transforms two lines (one, where two do not fit shared memory) of any
 // supported side: Stockham stages of radix 4, 2, 3, 5 and 7 between two buffers,
-// with the twiddles in a shared table.  What bounds it: latency (one or two waves
-// of blocks, a barrier a stage).
+// with the twiddles in a shared table.  What bounds it: latency (a few waves of
+// blocks, one or two an SM, a barrier a stage).  A hologram's two passes take 10 us
+// more than FP32 ones at side 512, 33 at 1024 and 245 at 2304; one line a block, 512
+// threads or a table made from fewer sincos did not shorten them.
 #include "rihvr_device.cuh"
 #include "rihvr_kernels.cuh"
 #include "rihvr_launch.cuh"
